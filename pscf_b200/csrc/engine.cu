@@ -38,6 +38,7 @@
 #include "kernels3l.cuh"
 #include "kernels3p.cuh"
 #include "basis.cuh"
+#include "kernels1.cuh"
 #include "am_graph.cuh"
 
 namespace pscfg {
@@ -1296,6 +1297,17 @@ static void sweep_steps(Engine &E, const SweepField<T> *dfl, int nf, int t0, int
         const size_t sm = Sweep2P<T, 64, 64>::smem_bytes();
         CK(allow_dyn_smem((const void *)k2p_sweep<T, 64, 64>));
         k2p_sweep<T, 64, 64><<<nf, 256, sm, E.st>>>(dfl, t0, t1);
+        E.launched();
+        return;
+    }
+    if (E.dim == 1 && !E.no_fixed_kernels && E.nr <= 128) {
+        // the step as a dense matrix held in registers; 128 points are the
+        // most whose matrix (128 KB) one CTA's registers hold
+        const int n = E.n[0];
+        const cx<double> *tw = (const cx<double> *)E.g64.rtw;
+        if (n <= 32) k1_sweep_dense<T, 32><<<nf, 128, 0, E.st>>>(dfl, n, t0, t1, tw);
+        else if (n <= 64) k1_sweep_dense<T, 64><<<nf, 256, 0, E.st>>>(dfl, n, t0, t1, tw);
+        else k1_sweep_dense<T, 128><<<nf, 512, 0, E.st>>>(dfl, n, t0, t1, tw);
         E.launched();
         return;
     }

@@ -1,0 +1,108 @@
+// kernels1.cuh -- 1-D sweeps of up to 128 points with the whole contour
+// step as one dense matrix.
+//
+// Within a block, step_exp (src/step_mod.f90:146-176) is the fixed linear
+// map q <- A q with
+//   A = (4 E2 C2 E1 C2 E2 - E1 C1 E1) / 3,
+// E1 = diag exp(-w ds/2), E2 = diag exp(-w ds/4) and C1, C2 the circulant
+// matrices of the k-space filters, c[d] = (1/N) sum_k ek(k) cos(2 pi k d/N).
+// On a line this short the six transforms of a step are nothing but latency
+// (a dozen barriers for 64 points), while A is N^2 <= 16384 numbers that fit
+// the registers of one CTA.  So a CTA forms A once per block (N^3
+// multiply-adds through shared memory) and then walks the contour with one
+// matrix-vector product and one barrier per step.
+#pragma once
+#include "kernels.cuh"
+
+namespace pscfg {
+
+// Four lanes per row, lane l holding the columns 8 j + 2 l and 8 j + 2 l + 1
+// (16-byte reads of q, four consecutive chunks per step, the same for every
+// row of a warp).  All arithmetic in FP64, also for FP32 slabs.
+// Bound: the serial chain of a step (shared-memory read, NMAX/16 dependent
+// multiply-adds, two shuffles, write, barrier).  64 points, 100 steps of a
+// diblock: 74 us, of which about half is the two blocks' matrices, against
+// 1132 us with k_sweep_plane; 192 fields: 108 us against 1166.
+// grid = nfields, 4 NMAX threads.
+template <typename T, int NMAX>
+__global__ void __launch_bounds__(4 * NMAX) k1_sweep_dense(const SweepField<T> *fields, int n, int t0, int t1,
+                                                           const cx<double> *__restrict__ tw)
+{
+    constexpr int J = NMAX / 8;
+    const SweepField<T> &f = fields[blockIdx.x];
+    __shared__ __align__(16) double qs[2][NMAX];
+    __shared__ double c1[2 * NMAX], c2[2 * NMAX], e1[NMAX], e2[NMAX];
+    int blk, src, dst;
+    if (!step_slices(f, t0, blk, src, dst)) return;
+    const int row = threadIdx.x >> 2, l = threadIdx.x & 3;
+    if (threadIdx.x < NMAX) {
+        const T *q = src_slice(f, src, n);
+        qs[0][threadIdx.x] = threadIdx.x < n ? (double)q[threadIdx.x] : 0.0;
+        qs[1][threadIdx.x] = 0.0;
+    }
+    double a[2 * J];
+    int cur = -1, p = 0;
+    for (int t = t0; t < t1; t++) {
+        if (!step_slices(f, t, blk, src, dst)) break;
+        if (blk != cur) {
+            cur = blk;
+            __syncthreads();
+            // circulants, twice in a row so that c[i - j + n] needs no modulus
+            for (int i = threadIdx.x; i < n; i += blockDim.x) {
+                double s1 = 0.0, s2 = 0.0;
+                for (int k = 0; k <= n / 2; k++) {
+                    const double w = (k == 0 || 2 * k == n) ? 1.0 : 2.0;
+                    const double c = w * tw[(k * i) % n].x;
+                    s1 += c * (double)f.ek1[blk][k];
+                    s2 += c * (double)f.ek2[blk][k];
+                }
+                c1[i] = c1[i + n] = s1 / n;
+                c2[i] = c2[i + n] = s2 / n;
+                e1[i] = (double)f.eo1[blk][i];
+                e2[i] = (double)f.eo2[blk][i];
+            }
+            __syncthreads();
+            const int i = row < n ? row : 0;
+#pragma unroll
+            for (int j = 0; j < 2 * J; j++) a[j] = 0.0;
+            for (int m = 0; m < n; m++) {
+                const double x = c2[i - m + n] * e1[m];
+#pragma unroll
+                for (int j = 0; j < 2 * J; j++) {
+                    const int col = min(8 * (j >> 1) + 2 * l + (j & 1), n - 1);
+                    a[j] += x * c2[m - col + n];
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 2 * J; j++) {
+                const int col = min(8 * (j >> 1) + 2 * l + (j & 1), n - 1);
+                a[j] = (4.0 * (e2[i] * a[j] * e2[col]) - e1[i] * c1[i - col + n] * e1[col]) / 3.0;
+            }
+        }
+        __syncthreads();
+        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+#pragma unroll
+        for (int j = 0; j < J; j++) {
+            // (columns beyond n meet the zeros kept there)
+            const double2 q = *(const double2 *)&qs[p][8 * j + 2 * l];
+            if (j & 1) {
+                s2 = fma(a[2 * j], q.x, s2);
+                s3 = fma(a[2 * j + 1], q.y, s3);
+            } else {
+                s0 = fma(a[2 * j], q.x, s0);
+                s1 = fma(a[2 * j + 1], q.y, s1);
+            }
+        }
+        double s = (s0 + s1) + (s2 + s3);
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        p ^= 1;
+        if (l == 0 && row < n) {
+            const T v = (T)s;
+            qs[p][row] = (double)v;
+            dst_slice(f, dst, n)[row] = v;
+        }
+    }
+}
+
+}  // namespace pscfg
