@@ -13,6 +13,9 @@
 namespace pscfg {
 
 #define PSCFG_MAXB 8
+#ifndef PSCFG_MAXM
+#define PSCFG_MAXM 4
+#endif
 
 // One contour sweep of one chain of one instance, in one direction.
 template <typename T>
@@ -464,6 +467,55 @@ __global__ void k_simpson(const SimpsonJob *jobs, const int *job_start, long nr)
             const SimpsonJob &J0 = jobs[j0];
             for (int a = 0; a < J0.n_monomer; a++) J0.rho[(long)a * nr + r] = acc[a];
         }
+    }
+}
+
+// k_simpson with SIMPSON_SPLIT threads per grid point, each summing every
+// SIMPSON_SPLIT-th slice of every block; the partial densities meet in
+// shared memory.  Bound: latency of the slice loads, which one thread per
+// point issues one after another (64 points, 101 slices: 13.9 us with
+// k_simpson, 5.2 here).  grid = (ceil(nr / 32), ninst), block (32, SIMPSON_SPLIT).
+constexpr int SIMPSON_SPLIT = 8;
+
+template <typename T>
+__global__ void __launch_bounds__(32 * SIMPSON_SPLIT) k_simpson_split(const SimpsonJob *jobs, const int *job_start, long nr)
+{
+    __shared__ double part[SIMPSON_SPLIT][PSCFG_MAXM][32];
+    const int j0 = job_start[blockIdx.y], j1 = job_start[blockIdx.y + 1];
+    if (j1 <= j0) return;
+    const int M = jobs[j0].n_monomer;
+    const long r = (long)blockIdx.x * 32 + threadIdx.x;
+    double acc[PSCFG_MAXM] = {0.0, 0.0, 0.0, 0.0};
+    if (r < nr) {
+        for (int jb = j0; jb < j1; jb++) {
+            const SimpsonJob &J = jobs[jb];
+            const T *qf = (const T *)J.qf, *qr = (const T *)J.qr;
+            const double Q = *J.Q;
+            const double phi = J.grand ? Q * exp(J.mu) : J.phi;
+            for (int b = 0; b < J.nblk; b++) {
+                const int ib = J.bgn[b], ie = J.bgn[b + 1];
+                double s = 0.0;
+#pragma unroll 4
+                for (int j = ib + (int)threadIdx.y; j <= ie; j += SIMPSON_SPLIT) {
+                    const double w = (j == ib || j == ie) ? 1.0 : (((j - ib) & 1) ? 4.0 : 2.0);
+                    s += w * ((double)qf[(long)j * nr + r] * (double)qr[(long)j * nr + r]);
+                }
+                s = phi * (s * J.bds[b] / 3.0 / J.length / Q);
+#pragma unroll
+                for (int a = 0; a < PSCFG_MAXM; a++)
+                    if (a == J.mon[b]) acc[a] += s;
+            }
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < PSCFG_MAXM; a++) part[threadIdx.y][a][threadIdx.x] = acc[a];
+    __syncthreads();
+    if (r >= nr) return;
+    for (int a = threadIdx.y; a < M; a += SIMPSON_SPLIT) {
+        double *rho = jobs[j0].rho + (long)a * nr + r;
+        double s = jobs[j0].accumulate ? *rho : 0.0;
+        for (int k = 0; k < SIMPSON_SPLIT; k++) s += part[k][a][threadIdx.x];
+        *rho = s;
     }
 }
 
