@@ -8,6 +8,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -29,21 +30,21 @@ def nvcc() -> str:
 def build(verbose: bool = False, extra=()) -> str:
     import tempfile
     os.makedirs(LIBDIR, exist_ok=True)
-    srcs = [os.path.join(CSRC, s) for s in SOURCES]
     common = [*ARCH, "-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC"]
-    with tempfile.TemporaryDirectory() as tmp:
-        objs = []
-        for name, flags in SEPARATE.items():
-            obj = os.path.join(tmp, name.replace(".cu", ".o"))
-            cmd = [nvcc(), *common, *flags, "-c", "-o", obj, os.path.join(CSRC, name), *extra]
-            if verbose:
-                print(" ".join(cmd))
-            subprocess.run(cmd, check=True)
-            objs.append(obj)
-        cmd = [nvcc(), *common, "-shared", "-o", LIB, *srcs, *objs, *extra]
+
+    def run(cmd):
         if verbose:
             print(" ".join(cmd))
         subprocess.run(cmd, check=True)
+
+    units = [(name, []) for name in SOURCES] + list(SEPARATE.items())
+    with tempfile.TemporaryDirectory() as tmp, ThreadPoolExecutor(max(1, os.cpu_count() or 1)) as pool:
+        objs = [os.path.join(tmp, name.replace(".cu", ".o")) for name, _ in units]
+        jobs = [pool.submit(run, [nvcc(), *common, *flags, "-c", "-o", obj, os.path.join(CSRC, name), *extra])
+                for (name, flags), obj in zip(units, objs)]
+        for j in jobs:
+            j.result()
+        run([nvcc(), *common, "-shared", "-o", LIB, *objs, *extra])
     return LIB
 
 

@@ -256,6 +256,9 @@ struct Engine {
         return p;
     }
 
+    // omega (or rho) of the whole batch, from inst[0]'s on
+    size_t fields_bytes() const { return sizeof(double) * (size_t)M * nr * inst.size(); }
+
     int cur = PSCFG_FP64;          // precision of the kernels being launched
     size_t tsize() const { return prec == PSCFG_FP32 ? sizeof(float) : sizeof(double); }
     const PlaneGeom &geom() const { return cur == PSCFG_FP32 ? g32 : g64; }
@@ -579,6 +582,10 @@ static void create_engine(Engine &E, const pscfg_system *sys, int n_inst, int pr
         E.ckK = std::max(1, (int)std::ceil(std::sqrt((double)ns_max)));
     }
     E.inst.resize(n_inst);
+    // the batch's fields lie one after another, as the host's arrays do, so
+    // that each crosses in one copy
+    const long fl = (long)E.M * E.nr;
+    double *omega_all = nullptr, *rho_all = nullptr;
     for (int i = 0; i < n_inst; i++) {
         pscfg_system s = sys[i];
         for (int d = s.dim; d < 3; d++) s.n[d] = 1;
@@ -587,8 +594,12 @@ static void create_engine(Engine &E, const pscfg_system *sys, int n_inst, int pr
         Inst &I = E.inst[i];
         I.sys = s;
         I.prec_now = (precision == PSCFG_FP32) ? PSCFG_FP32 : PSCFG_FP64;
-        I.omega = (double *)E.dalloc(sizeof(double) * E.M * E.nr);
-        I.rho = (double *)E.dalloc(sizeof(double) * E.M * E.nr);
+        if (i == 0) {
+            omega_all = (double *)E.dalloc(sizeof(double) * fl * n_inst);
+            rho_all = (double *)E.dalloc(sizeof(double) * fl * n_inst);
+        }
+        I.omega = omega_all + i * fl;
+        I.rho = rho_all + i * fl;
         I.ksq = (double *)E.dalloc(sizeof(double) * E.nk);
         I.wdgsq = (double *)E.dalloc(sizeof(double) * PSCFG_MAXCP * E.nk);
         I.Qdev = (double *)E.dalloc(sizeof(double) * PSCFG_MAXC);
@@ -2439,27 +2450,44 @@ static void am_begin(Engine &E, AmRun &R, const pscfg_am_param &prm)
     // symmetric initial guess, then the first density (src/iterate_mod.fp.f90:1123)
     symmetrize_omega(E, all);
     density_all(E, all);
-    // uniform component of omega (set_omega_uniform, src/scf_mod.fp.f90:724-750)
-    std::vector<double> w(fl);
+    // uniform component of omega (set_omega_uniform, src/scf_mod.fp.f90:724-750),
+    // and the first history entry
+    std::vector<const double *> wp;
+    std::vector<UniformJob> uj;
     for (int i = 0; i < ninst; i++) {
         Inst &I = E.inst[i];
-        CK(cudaMemcpyAsync(w.data(), I.omega, sizeof(double) * fl, cudaMemcpyDeviceToHost, E.st));
-        CK(cudaStreamSynchronize(E.st));
         double phi_mon[PSCFG_MAXM] = {0};
         for (int c = 0; c < I.sys.n_chain; c++)
             for (int b = 0; b < I.sys.n_block[c]; b++)
                 phi_mon[I.sys.block_monomer[c][b]] += I.sys.phi_chain[c] * I.sys.block_length[c][b] / I.length[c];
         for (int sv = 0; sv < I.sys.n_solvent; sv++) phi_mon[I.sys.solvent_monomer[sv]] += I.sys.phi_solvent[sv];
-        for (int a = 0; a < E.M && I.sys.ensemble == 0; a++) {
-            double w0 = 0;
-            for (int b = 0; b < E.M; b++) w0 = w0 + I.sys.chi[a][b] * phi_mon[b];
-            double m = 0;
-            for (long r = 0; r < E.nr; r++) m += w[a * E.nr + r];
-            m /= (double)E.nr;
-            for (long r = 0; r < E.nr; r++) w[a * E.nr + r] += w0 - m;
+        UniformJob j;
+        std::memset(&j, 0, sizeof(j));
+        j.omega = I.omega;
+        j.hist = I.om_hist;
+        j.mean = E.d_small + (size_t)i * E.M;
+        j.M = E.M;
+        j.shift = I.sys.ensemble == 0;
+        for (int a = 0; a < E.M; a++) {
+            for (int b = 0; b < E.M; b++) j.w0[a] = j.w0[a] + I.sys.chi[a][b] * phi_mon[b];
+            wp.push_back(I.omega + a * E.nr);
         }
-        CK(cudaMemcpyAsync(I.omega, w.data(), sizeof(double) * fl, cudaMemcpyHostToDevice, E.st));
-        CK(cudaMemcpyAsync(I.om_hist, I.omega, sizeof(double) * fl, cudaMemcpyDeviceToDevice, E.st));
+        uj.push_back(j);
+    }
+    {
+        const int nj = (int)wp.size(), nct = red_ctas(E.nr, nj);
+        const double **dwp = (const double **)E.upload(wp, 0);
+        UniformJob *duj = E.upload(uj, (wp.size() * sizeof(void *) + 255) / 256 * 256);
+        double *part = E.part((size_t)nct * nj);
+        k_partial_sum<double><<<dim3(nct, nj), 256, 0, E.st>>>(dwp, E.nr, part);
+        E.launched();
+        k_final_sum<<<(unsigned)((nj + 127) / 128), 128, 0, E.st>>>(part, nct, (double)E.nr, E.d_small, nj);
+        E.launched();
+        k_omega_uniform<<<dim3(red_ctas(E.nr, ninst), ninst), 256, 0, E.st>>>(duj, E.nr);
+        E.launched();
+    }
+    for (int i = 0; i < ninst; i++) {
+        Inst &I = E.inst[i];
         AmState &st = R.st[i];
         st.gram.assign((size_t)S * S, 0.0);
         st.devcp.assign(S, std::vector<double>(PSCFG_MAXCP, 0.0));
@@ -4072,19 +4100,15 @@ static int density_common(pscfg_engine *e, const double *omega, double *rho, dou
 {
     ABI_BEGIN
     Engine &E = e->E;
-    const long fl = (long)E.M * E.nr;
     const int ni = (int)E.inst.size();
-    for (int i = 0; i < ni; i++)
-        CK(cudaMemcpyAsync(E.inst[i].omega, omega + (long)i * fl, sizeof(double) * fl,
-                           device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, E.st));
+    CK(cudaMemcpyAsync(E.inst[0].omega, omega, E.fields_bytes(),
+                       device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, E.st));
     std::vector<int> all(ni);
     for (int i = 0; i < ni; i++) all[i] = i;
     density_all(E, all);
-    if (rho) {
-        for (int i = 0; i < ni; i++)
-            CK(cudaMemcpyAsync(rho + (long)i * fl, E.inst[i].rho, sizeof(double) * fl,
-                               device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, E.st));
-    }
+    if (rho)
+        CK(cudaMemcpyAsync(rho, E.inst[0].rho, E.fields_bytes(), device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
+                           E.st));
     CK(cudaStreamSynchronize(E.st));
     for (int i = 0; i < ni; i++) {
         if (q)
@@ -4117,10 +4141,13 @@ int pscfg_stress(pscfg_engine *e, double *stress)
     std::vector<int> all(ni);
     for (int i = 0; i < ni; i++) all[i] = i;
     stress_all(E, all);
-    for (int i = 0; i < ni; i++)
-        CK(cudaMemcpyAsync(stress + (long)i * PSCFG_MAXCP, E.inst[i].stress_dev, sizeof(double) * PSCFG_MAXCP,
-                           cudaMemcpyDeviceToHost, E.st));
+    std::vector<CopyJob> cj;
+    double *dst = E.dstage + (size_t)E.hpin_inst * 16;
+    for (int i = 0; i < ni; i++) cj.push_back(CopyJob{E.inst[i].stress_dev, dst + (size_t)i * 8, PSCFG_MAXCP});
+    copy_list(E, cj, 8);
+    CK(cudaMemcpyAsync(E.hst(0), dst, sizeof(double) * 8 * ni, cudaMemcpyDeviceToHost, E.st));
     CK(cudaStreamSynchronize(E.st));
+    for (int i = 0; i < ni; i++) std::memcpy(stress + (long)i * PSCFG_MAXCP, E.hst(i), sizeof(double) * PSCFG_MAXCP);
     for (int i = 0; i < ni; i++)
         for (int b = E.inst[i].cell.ncp; b < PSCFG_MAXCP; b++) stress[(long)i * PSCFG_MAXCP + b] = 0.0;
     ABI_END(e)
@@ -4151,18 +4178,13 @@ int pscfg_free_energy(pscfg_engine *e, double *out, double *mu_chain)
 
 static void load_omega(Engine &E, const double *omega)
 {
-    const long fl = (long)E.M * E.nr;
-    for (size_t i = 0; i < E.inst.size(); i++)
-        CK(cudaMemcpyAsync(E.inst[i].omega, omega + (long)i * fl, sizeof(double) * fl, cudaMemcpyHostToDevice, E.st));
+    CK(cudaMemcpyAsync(E.inst[0].omega, omega, E.fields_bytes(), cudaMemcpyHostToDevice, E.st));
 }
 
 static void store_fields(Engine &E, double *omega, double *rho)
 {
-    const long fl = (long)E.M * E.nr;
-    for (size_t i = 0; i < E.inst.size(); i++) {
-        if (omega) CK(cudaMemcpyAsync(omega + (long)i * fl, E.inst[i].omega, sizeof(double) * fl, cudaMemcpyDeviceToHost, E.st));
-        if (rho) CK(cudaMemcpyAsync(rho + (long)i * fl, E.inst[i].rho, sizeof(double) * fl, cudaMemcpyDeviceToHost, E.st));
-    }
+    if (omega) CK(cudaMemcpyAsync(omega, E.inst[0].omega, E.fields_bytes(), cudaMemcpyDeviceToHost, E.st));
+    if (rho) CK(cudaMemcpyAsync(rho, E.inst[0].rho, E.fields_bytes(), cudaMemcpyDeviceToHost, E.st));
     CK(cudaStreamSynchronize(E.st));
 }
 

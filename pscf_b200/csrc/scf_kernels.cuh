@@ -310,6 +310,29 @@ static __global__ void k_am_dev(const AmJob *jobs, long nr, double *part)
     }
 }
 
+// Start of a run: the uniform component of each omega_a set to w0[a]
+// (shift != 0), and omega copied to the first history entry.
+struct UniformJob {
+    double *omega, *hist;
+    const double *mean;       // [M] device
+    double w0[PSCFG_MAXM];
+    int M, shift;
+};
+
+static __global__ void k_omega_uniform(const UniformJob *jobs, long nr)
+{
+    const UniformJob &J = jobs[blockIdx.y];
+    for (int a = 0; a < J.M; a++) {
+        const double d = J.shift ? J.w0[a] - J.mean[a] : 0.0;
+        double *w = J.omega + (long)a * nr, *h = J.hist + (long)a * nr;
+        for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < nr; r += (long)gridDim.x * blockDim.x) {
+            const double v = J.shift ? w[r] + d : w[r];
+            w[r] = v;
+            h[r] = v;
+        }
+    }
+}
+
 // Subtract the mean of each dev_a and return partial max |dev|.
 struct AmFix {
     double *dev;
