@@ -308,9 +308,8 @@ int pscfg_propagate(pscfg_engine *e, int inst, const double *omega_m, double b, 
  * 512 n3 bytes each.  Other grids are rejected with PSCFG_EINVAL, before
  * any GPU work is queued, and a message from pscfg_last_error(NULL).  The
  * first call on a device does a one-time set-up with that device current:
- * it looks up the array's device address (cudaGetSymbolAddress) and copies
- * the codelet constants to the device (cudaMemcpyToSymbol).  After that a
- * call queues kernel launches only (no host-device copies).  All calls
+ * it looks up the array's device address (cudaGetSymbolAddress).  After
+ * that a call queues kernel launches only (no host-device copies).  All calls
  * on a device share the array: calls whose GPU work overlaps (other host
  * threads, or streams with no ordering between them) race on it.  Each
  * call writes every scratch entry it reads, so nothing carries over from
@@ -363,13 +362,13 @@ long pscfg_steps_per_density(const pscfg_engine *e);
 /* Kernel launches issued by this engine since creation (all streams). */
 long pscfg_launch_count(const pscfg_engine *e);
 
-/* Planes per CTA that the 3-D register sweep of this engine's grid uses for
- * a sweep of n_fields fields in FP64 (fp32 != 0: FP32), as measured by the
- * engine (one timed trial sweep per candidate before the first real sweep
- * of each class of field counts -- up to the same power of two -- the
+/* Planes per CTA that the 3-D sweep of this engine's grid (16^3, 32^3) uses
+ * for n_fields fields in FP64 (fp32 != 0: FP32).  FP64: by the launch size.
+ * FP32, and FP64 with PSCFG_PLANES set: as measured by the engine for its
+ * register sweep (one timed trial sweep per candidate before the first real
+ * sweep of each class of field counts -- up to the same power of two -- the
  * fastest kept for the process); -1 when the thread-block-cluster sweep
- * (32^3, FP64) was the fastest; 0 while undecided or for grids without the
- * register sweep (16^3, 32^3). */
+ * (32^3, FP64) was the fastest; 0 while undecided or for other grids. */
 int pscfg_sweep_planes(const pscfg_engine *e, int n_fields, int fp32);
 
 #ifdef __cplusplus

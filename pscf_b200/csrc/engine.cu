@@ -36,9 +36,9 @@
 #include "kernels3x.cuh"
 #include "response.cuh"
 #include "kernels3l.cuh"
-#include "kernels3p.cuh"
 #include "basis.cuh"
 #include "kernels1.cuh"
+#include "sweep_rx.h"
 #include "am_graph.cuh"
 
 namespace pscfg {
@@ -153,7 +153,7 @@ struct Engine {
     bool smem_fft = false;           // shared-memory x-y column passes (PSCFG_SMEM_FFT=1)
     bool no_graphs = false;          // launch the 3-D sweeps directly (PSCFG_NO_GRAPHS=1)
     bool line_step = false;          // line-pass 3-D step even where the plane kernels fit (PSCFG_LINE_STEP=1)
-    int plane_p = 1;                 // shared-memory plane kernels (kernels3p.cuh) for 64x128x224 and 64^3; 0: off (PSCFG_PLANE_P)
+    int plane_p = 1;                 // 3-D kernels of plane_rx.cuh; 0: the older kernels (PSCFG_PLANE_P)
     int planes = 0;                  // planes per CTA of the register sweep, 0 = by launch size (PSCFG_PLANES)
     // CUDA graphs of 3-D sweeps, keyed by descriptor address, field and step count
     struct SweepGraph {
@@ -174,6 +174,7 @@ struct Engine {
 
     // FFT plan / twiddle tables
     PlaneGeom g64, g32;
+    RxPlan rx;                   // shapes and tables of the plane_rx.cuh kernels
     std::vector<void *> allocs;
 
     // descriptor scratch (device), grown on demand
@@ -337,6 +338,13 @@ struct Engine {
         }
         return d_part;
     }
+    // n kernels queued by a sweep_rx.h launch function (n < 0: one failed)
+    bool launched_n(int n)
+    {
+        launched();
+        launches += n - 1;
+        return n > 0;
+    }
     void launched(cudaError_t e = cudaGetLastError())
     {
         launches++;
@@ -385,48 +393,8 @@ static void make_geom(Engine &E, PlaneGeom &g)
     g.rtw = twiddle_table<T>(E, g.n1);
 }
 
-// W_N^m tables of the plane kernels (kernels3p.cuh), FP64 and FP32.
-template <int N>
-static void upload_ptw(const void *sym_d, const void *sym_f)
-{
-    double d[2][N];
-    float f[2][N];
-    for (int m = 0; m < N; m++) {
-        long double a = -2.0L * 3.14159265358979323846264338327950288L * m / (long double)N;
-        d[0][m] = (double)cosl(a);
-        d[1][m] = (double)sinl(a);
-        f[0][m] = (float)cosl(a);
-        f[1][m] = (float)sinl(a);
-    }
-    CK(cudaMemcpyToSymbol(sym_d, d, sizeof(d)));
-    CK(cudaMemcpyToSymbol(sym_f, f, sizeof(f)));
-}
-
-static void upload_p_twiddles()
-{
-    upload_ptw<32>(c_ptw32, c_ptw32f);
-    upload_ptw<64>(c_ptw64, c_ptw64f);
-    upload_ptw<128>(c_ptw128, c_ptw128f);
-    upload_ptw<224>(c_ptw224, c_ptw224f);
-}
-
 static void upload_dft_constants()
 {
-    // row 0: cos(2 pi m/R), row 1: sin(2 pi m/R); the codelet forms
-    // W = (cos, S*sin) with S = -1 forward, +1 inverse.
-    double t5[2][5], t7[2][7];
-    for (int m = 0; m < 5; m++) {
-        long double a = 2.0L * 3.14159265358979323846264338327950288L * m / 5.0L;
-        t5[0][m] = (double)cosl(a);
-        t5[1][m] = (double)sinl(a);
-    }
-    for (int m = 0; m < 7; m++) {
-        long double a = 2.0L * 3.14159265358979323846264338327950288L * m / 7.0L;
-        t7[0][m] = (double)cosl(a);
-        t7[1][m] = (double)sinl(a);
-    }
-    CK(cudaMemcpyToSymbol(c_dft5, t5, sizeof(t5)));
-    CK(cudaMemcpyToSymbol(c_dft7, t7, sizeof(t7)));
     double w64[2][64];
     for (int m = 0; m < 64; m++) {
         long double a = -2.0L * 3.14159265358979323846264338327950288L * m / 64.0L;
@@ -434,7 +402,6 @@ static void upload_dft_constants()
         w64[1][m] = (double)sinl(a);
     }
     CK(cudaMemcpyToSymbol(c_w64, w64, sizeof(w64)));
-    upload_p_twiddles();
 }
 
 // ---------------------------------------------------------------------
@@ -567,6 +534,19 @@ static void create_engine(Engine &E, const pscfg_system *sys, int n_inst, int pr
     upload_dft_constants();
     make_geom<double>(E, E.g64);
     if (precision != PSCFG_FP64) make_geom<float>(E, E.g32);
+    {
+        std::vector<RxCol> cols(E.n[0] / 2 + 1);
+        if (rx_shape(E.dim, E.n, E.rx, cols.data())) {
+            RxCol *d = (RxCol *)E.dalloc(cols.size() * sizeof(RxCol));
+            CK(cudaMemcpy(d, cols.data(), cols.size() * sizeof(RxCol), cudaMemcpyHostToDevice));
+            for (int k = 0; k < 2; k++) {
+                const PlaneGeom &g = k ? E.g32 : E.g64;
+                E.rx.tb[k] = RxTables{g.rtw, g.col.tw, d};
+                E.rx.zc[k].cols = d;
+                E.rx.zc[k].twz = g.zp.tw;
+            }
+        }
+    }
 
     const size_t ts = E.tsize();
     if (E.ckpt) {
@@ -942,33 +922,77 @@ static bool sweep3r(Engine &E, const SweepField<T> *dfl, int nf, int ns_max, int
     return false;
 }
 
-// Whether the sweep of this engine runs the plane kernels (kernels3p.cuh).
-static bool plane_kernels_apply(const Engine &E)
+// Whether the 3-D steps and stress of this engine run the plane_rx.cuh
+// kernels.  The register-column kernels (kernels3c.cuh) keep 16^3, where
+// their whole columns in registers win (density + stress of 1 / 16 / 64
+// diblocks: 1.94 / 2.40 / 4.16 ms against 2.72 / 3.11 / 4.99), not 32^3 (4 /
+// 16: 3.58 / 6.36 ms against 2.55 / 5.29).  FP32 keeps them at 32^3 too: the
+// mixed-precision switch of the Anderson runs was tuned on their rounding
+// (with packed FP32 columns one of 64 BCC solves left its basin).
+template <typename T>
+static bool rx3_applies(const Engine &E)
 {
     if (E.dim != 3 || E.no_fixed_kernels || E.smem_fft || E.cluster_step || E.line_step || E.plane_p == 0) return false;
-    const int a = E.n[0], b = E.n[1], c = E.n[2];
-    return (a == 64 && b == 128 && c == 224) || (a == 64 && b == 64 && c == 64);
+    const bool cube = E.n[0] == E.n[1] && E.n[1] == E.n[2];
+    if (cube && (E.n[0] == 16 || (E.n[0] == 32 && (sizeof(T) == 4 || E.planes != 0)))) return false;
+    return rx3_fits<T>(E.rx);
 }
 
-// Position p of a forward four-step transform of length N (Split<N> of
-// fft_ct.cuh / kernels3p.cuh) -> frequency index.
-__host__ __device__ static inline int host_iperm(int N, int p)
+// A whole 3-D sweep with the plane_rx.cuh kernels.  The fields of a group
+// run as two independent kernel chains on two streams, so that each launch's
+// last, partly empty wave overlaps the other chain's work; a batch whose
+// step scratch (both spectra, the block's table, two slices) overflows the L2 goes in groups
+// that fit it, each group through the whole contour (32^3 x 64 instances:
+// sweep 21.1 ms in groups of 32 or 64 fields, 23.1 at once, 25.5 in groups
+// of 16, whose launches no longer fill the GPU).
+template <typename T>
+static bool sweep3v(Engine &E, const SweepField<T> *dfl, int nf, int ns_max, int t0 = 0)
 {
-    int P = 1, Q = 1;
-    switch (N) {
-    case 32: P = 4; Q = 8; break;
-    case 64: P = 8; Q = 8; break;
-    case 128: P = 8; Q = 16; break;
-    case 224: P = 16; Q = 14; break;
-    default: P = N; Q = 1; break;
-    }
-    return p / Q + P * (p % Q);
+    if (!rx3_applies<T>(E)) return false;
+    const long field_bytes = (long)sizeof(T) * (4 * E.nk + 3 * E.nr);
+    const int fit = (int)std::max<long>(2, ((long)80 << 20) / field_bytes);
+    auto step = [&](const SweepField<T> *d, int n, cudaStream_t st, int t) {
+        E.launched_n(t < t0 ? rx3_first<T>(E.rx, st, d, n, t0) : rx3_step<T>(E.rx, st, d, n, t));
+    };
+    auto emit = [&]() {
+        if (nf < 2 || E.no_branch) {
+            for (int t = t0 - 1; t < ns_max; t++) step(dfl, nf, E.st, t);
+            return;
+        }
+        CK(cudaEventRecord(E.ev_fork, E.st));
+        CK(cudaStreamWaitEvent(E.st2, E.ev_fork, 0));
+        const int groups = (nf + fit - 1) / fit;
+        for (int g = 0; g < groups; g++) {
+            const int a = (int)((long)nf * g / groups), n = (int)((long)nf * (g + 1) / groups) - a, h = (n + 1) / 2;
+            for (int t = t0 - 1; t < ns_max; t++) {
+                step(dfl + a, h, E.st, t);
+                if (n > h) step(dfl + a + h, n - h, E.st2, t);
+            }
+        }
+        CK(cudaEventRecord(E.ev_join, E.st2));
+        CK(cudaStreamWaitEvent(E.st, E.ev_join, 0));
+    };
+    // launches longer than their cost on the host need no graph, whose
+    // capture and instantiation (~25 us a launch) the first sweep of an
+    // engine would pay (32^3 x 64: 2448 launches, 65 ms)
+    if ((long)std::min(fit, nf) * E.nr >= (1L << 20)) emit();
+    else graph_sweep(E, dfl, nf, ns_max, (int)sizeof(T), t0, emit, 200);
+    return true;
+}
+
+// Whether the z passes take the k-space filters as products of 1-D factors
+// (orthogonal cells): it saves 1/4 of their reads, and costs the host
+// 2 (n1/2 + n2 + n3) exponentials per block, too many for batches of small
+// grids.
+static bool ek_factors_apply(const Engine &E)
+{
+    return E.nr >= (1L << 18) && (E.cur == PSCFG_FP32 ? rx3_applies<float>(E) : rx3_applies<double>(E));
 }
 
 // 1-D factors of exp(-lap k^2/6) and exp(-lap k^2/12) (lap = ds b^2) of an
-// orthogonal cell over the plane kernels' spectrum positions: x (N1/2 + 1),
-// y (N2) and z (N3), each index folded to its minimum image (G_to_bz,
-// src/grid_mod.f90:225-283, along each axis).  Appends 2 (N1/2+1+N2+N3).
+// orthogonal cell: x (N1/2 + 1), y (N2) and z (N3), each index folded to its
+// minimum image (G_to_bz, src/grid_mod.f90:225-283, along each axis).
+// Appends 2 (N1/2+1+N2+N3).
 template <typename T>
 static void append_ek_factors(const Engine &E, const Cell &cell, double lap, std::vector<T> &out)
 {
@@ -981,9 +1005,9 @@ static void append_ek_factors(const Engine &E, const Cell &cell, double lap, std
     };
     for (int div : {6, 12}) {
         const long double c = (long double)lap / div;
-        for (int xp = 0; xp <= M; xp++) out.push_back((T)expl(-c * g2(0, xp < M ? host_iperm(M, xp) : M)));
-        for (int yp = 0; yp < n2; yp++) out.push_back((T)expl(-c * g2(1, host_iperm(n2, yp))));
-        for (int zp = 0; zp < n3; zp++) out.push_back((T)expl(-c * g2(2, host_iperm(n3, zp))));
+        for (int k = 0; k <= M; k++) out.push_back((T)expl(-c * g2(0, k)));
+        for (int k = 0; k < n2; k++) out.push_back((T)expl(-c * g2(1, k)));
+        for (int k = 0; k < n3; k++) out.push_back((T)expl(-c * g2(2, k)));
     }
 }
 
@@ -1010,93 +1034,20 @@ static __global__ void k_ek_factors(const EkfJob *jobs, int n1, int n2, int n3)
         if (j <= M) {
             axis = 0;
             n = n1;
-            k = j < M ? host_iperm(M, j) : M;
+            k = j;
         } else if (j < M + 1 + n2) {
             axis = 1;
             n = n2;
-            k = host_iperm(n2, j - M - 1);
+            k = j - M - 1;
         } else {
             axis = 2;
             n = n3;
-            k = host_iperm(n3, j - M - 1 - n2);
+            k = j - M - 1 - n2;
         }
         const double kf = (k > n / 2) ? (double)(k - n) : (double)k;
         const double g = J.G[axis * 3 + axis] * kf;
         out[i] = (T)exp(-c * g * g);
     }
-}
-
-// A whole 3-D sweep with the shared-memory plane kernels of kernels3p.cuh
-// (64 x 128 x 224 and 64^3; PSCFG_PLANE_P=0 selects the other kernels:
-// run-time shaped at 64 x 128 x 224, k3c at 64^3).  Returns false where not
-// applicable.  64^3, 4 instances, FP64 sweep: 61.3k field-steps/s against
-// 30.8k with the k3c kernels; 64 x 128 x 224, 1 instance: 8.0k against 2.5k.
-template <typename T>
-static bool sweep3p(Engine &E, const SweepField<T> *dfl, int nf, int ns_max, int t0 = 0)
-{
-    if (E.no_fixed_kernels || E.smem_fft || E.cluster_step || E.line_step || E.plane_p == 0) return false;
-    auto run = [&](auto n1c, auto n2c, auto n3c, auto tcc) {
-        constexpr int N1 = decltype(n1c)::value, N2 = decltype(n2c)::value, N3 = decltype(n3c)::value;
-        constexpr int TC = decltype(tcc)::value;
-        using PL = PlaneP<T, N1, N2>;
-        const size_t smp = sizeof(cx<T>) * PL::PS, smz = sizeof(cx<T>) * N3 * TC;
-        CK(allow_dyn_smem((const void *)k3p_fwd_pair<T, N1, N2, N3>));
-        CK(allow_dyn_smem((const void *)k3p_mid<T, N1, N2, N3>));
-        CK(allow_dyn_smem((const void *)k3p_final_fwd<T, N1, N2, N3>));
-        CK(allow_dyn_smem((const void *)k3p_zconv<T, N1, N2, N3, TC>));
-        const PlaneGeom g = E.geom();
-        const unsigned ztiles = (unsigned)(PL::PS / TC);
-        int dev = 0, nsm = 148;
-        CK(cudaGetDevice(&dev));
-        CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        const int pf = 2 * nsm;   // CTAs of k3p_zconv resident at once (2 per SM)
-        // a small batch's fields run as two independent kernel chains (the
-        // qf and qr sweeps of one instance, for instance), so that each
-        // launch's last, partly empty wave overlaps the other chain's work
-        const int h = (nf >= 2 && nf <= 8 && !E.no_branch) ? nf / 2 : 0;
-        auto step = [&](const SweepField<T> *d, int n, cudaStream_t s, int t) {
-            if (t < t0) {
-                k3p_fwd_pair<T, N1, N2, N3><<<dim3(N3, n), 256, smp, s>>>(d, g, t0);
-                E.launched();
-                return;
-            }
-            k3p_zconv<T, N1, N2, N3, TC><<<dim3(ztiles, n, 2), 256, smz, s>>>(d, g, t, 3, pf);
-            E.launched();
-            k3p_mid<T, N1, N2, N3><<<dim3(N3, n, 2), 256, smp, s>>>(d, g, t);
-            E.launched();
-            k3p_zconv<T, N1, N2, N3, TC><<<dim3(ztiles, n, 1), 256, smz, s>>>(d, g, t, 2, pf);
-            E.launched();
-            k3p_final_fwd<T, N1, N2, N3><<<dim3(N3, n), 256, smp, s>>>(d, g, t);
-            E.launched();
-        };
-        auto emit = [&]() {
-            if (h == 0) {
-                for (int t = t0 - 1; t < ns_max; t++) step(dfl, nf, E.st, t);
-                return;
-            }
-            CK(cudaEventRecord(E.ev_fork, E.st));
-            CK(cudaStreamWaitEvent(E.st2, E.ev_fork, 0));
-            for (int t = t0 - 1; t < ns_max; t++) {
-                step(dfl, h, E.st, t);
-                step(dfl + h, nf - h, E.st2, t);
-            }
-            CK(cudaEventRecord(E.ev_join, E.st2));
-            CK(cudaStreamWaitEvent(E.st, E.ev_join, 0));
-        };
-        graph_sweep(E, dfl, nf, ns_max, (int)sizeof(T), t0, emit);
-    };
-    const int a = E.n[0], b = E.n[1], c = E.n[2];
-    if (a == 64 && b == 128 && c == 224) {
-        run(std::integral_constant<int, 64>(), std::integral_constant<int, 128>(), std::integral_constant<int, 224>(),
-            std::integral_constant<int, 16>());
-        return true;
-    }
-    if (a == 64 && b == 64 && c == 64) {
-        run(std::integral_constant<int, 64>(), std::integral_constant<int, 64>(), std::integral_constant<int, 64>(),
-            std::integral_constant<int, 32>());
-        return true;
-    }
-    return false;
 }
 
 // One 3-D MDE step as line passes (kernels3l.cuh), for grids with an even
@@ -1233,7 +1184,7 @@ static void run_sweeps(Engine &E, const std::vector<int> &act)
     std::vector<T> ekf;
     std::vector<EkfJob> ekj;
     const int L3 = (int)(E.n[0] / 2 + 1) + E.n[1] + E.n[2];
-    if (plane_kernels_apply(E)) {
+    if (ek_factors_apply(E)) {
         bool ortho = true;
         for (int i : act) {
             if (E.amg) {
@@ -1303,14 +1254,7 @@ static void sweep_steps(Engine &E, const SweepField<T> *dfl, int nf, int t0, int
 {
     const PlaneGeom &g = E.geom();
     const int ns_max = t1;
-    if (E.dim == 2 && !E.no_fixed_kernels && E.n[0] == 64 && E.n[1] == 64) {
-        // fixed-shape whole-sweep kernel: tables and q in shared memory
-        const size_t sm = Sweep2P<T, 64, 64>::smem_bytes();
-        CK(allow_dyn_smem((const void *)k2p_sweep<T, 64, 64>));
-        k2p_sweep<T, 64, 64><<<nf, 256, sm, E.st>>>(dfl, t0, t1);
-        E.launched();
-        return;
-    }
+    if (E.dim == 2 && !E.no_fixed_kernels && E.launched_n(rx2_sweep<T>(E.rx, E.st, dfl, nf, t0, t1))) return;
     if (E.dim == 1 && !E.no_fixed_kernels && E.nr <= 128) {
         // the step as a dense matrix held in registers; 128 points are the
         // most whose matrix (128 KB) one CTA's registers hold
@@ -1329,7 +1273,7 @@ static void sweep_steps(Engine &E, const SweepField<T> *dfl, int nf, int t0, int
         // one CTA per field: a sweep of few fields is bound by the latency of
         // its FFT phases, which more warps hide (64 x 64 with this kernel,
         // one instance: 5.30 -> 4.28 ms per density with 512 threads instead
-        // of 256; k2p_sweep above: 2.16 ms)
+        // of 256)
         int threads = (int)std::min<long>(512, std::max<long>(32, ((E.nr / 2 + 31) / 32) * 32));
         k_sweep_plane<T><<<nf, threads, sm, E.st>>>(dfl, g, t0, t1);
         E.launched();
@@ -1345,8 +1289,8 @@ static void sweep_steps(Engine &E, const SweepField<T> *dfl, int nf, int t0, int
         const long P = (long)g.n1h * g.n2;
         const int ntile = (int)((P + Z_TILE - 1) / Z_TILE);
         const int txy = 256, tz = 256;
+        if (sweep3v<T>(E, dfl, nf, ns_max, t0)) return;
         if (sweep3r<T>(E, dfl, nf, ns_max, t0)) return;
-        if (sweep3p<T>(E, dfl, nf, ns_max, t0)) return;
         for (int t = t0; t < ns_max; t++) {
             if (step3_fixed<T>(E, dfl, nf, t)) continue;
             if (step3l<T>(E, dfl, nf, t)) continue;
@@ -1562,7 +1506,7 @@ static void ckpt_tables(Engine &E, const std::vector<int> &act, std::vector<cons
     ekf_of.clear();
     std::vector<T> ekf;
     const int L3 = (int)(E.n[0] / 2 + 1) + E.n[1] + E.n[2];
-    bool sep = plane_kernels_apply(E);
+    bool sep = ek_factors_apply(E);
     for (int i : act)
         for (int a = 0; a < 3; a++)
             for (int b2 = 0; b2 < 3; b2++)
@@ -1930,32 +1874,11 @@ static void stress3r(Engine &E, const StressJob<T> *dj, int s0, int cnt)
     E.launched();
 }
 
-// The stress slice pass with the plane kernels (kernels3p.cuh), for the
-// shapes whose sweep uses them.
-template <typename T, int N1, int N2, int N3, int TC>
-static void stress3p(Engine &E, const StressJob<T> *dj, int s0, int cnt)
-{
-    using PL = PlaneP<T, N1, N2>;
-    const size_t smp = sizeof(cx<T>) * PL::PS, smz = 2 * sizeof(cx<T>) * N3 * TC;
-    CK(allow_dyn_smem((const void *)k3p_stress_xy<T, N1, N2, N3>));
-    CK(allow_dyn_smem((const void *)k3p_stress_z<T, N1, N2, N3, TC>));
-    const int ntile = PL::PS / TC;
-    k3p_stress_xy<T, N1, N2, N3><<<dim3(N3, cnt, 2), 256, smp, E.st>>>(dj, s0, (cx<T> *)E.spec);
-    E.launched();
-    k3p_stress_z<T, N1, N2, N3, TC><<<dim3(ntile, cnt), 256, smz, E.st>>>(dj, s0, (const cx<T> *)E.spec, E.stress_part);
-    E.launched();
-    k3_stress_sum<T><<<cnt, 32, 0, E.st>>>(dj, s0, ntile, E.stress_part);
-    E.launched();
-}
-
 template <typename T>
 static bool stress3_fixed(Engine &E, const StressJob<T> *dj, int s0, int cnt)
 {
     if (E.no_fixed_kernels) return false;
     const int a = E.n[0], b = E.n[1], c = E.n[2];
-    const bool pk = !(E.smem_fft || E.cluster_step || E.line_step || E.plane_p == 0);
-    if (pk && a == 64 && b == 128 && c == 224) { stress3p<T, 64, 128, 224, 8>(E, dj, s0, cnt); return true; }
-    if (pk && a == 64 && b == 64 && c == 64) { stress3p<T, 64, 64, 64, 16>(E, dj, s0, cnt); return true; }
     if (a == 32 && b == 32 && c == 32) {
         if (E.smem_fft) stress3c<T, 32, 32, 32, 8>(E, dj, s0, cnt);
         else stress3r<T, 32, 32, 32, 4>(E, dj, s0, cnt);
@@ -2025,6 +1948,41 @@ static bool slice_dots_r(Engine &E, const StressJob<T> *dj, int njobs, int maxs)
     return false;
 }
 
+// All jobs of slice_dots with the plane_rx.cuh kernels, in chunks of slices
+// whose spectra take at most 1 GB.
+template <typename T>
+static bool slice_dots_v(Engine &E, const StressJob<T> *dj, int njobs, int maxs)
+{
+    const int ntile = rx3_stress_tiles<T>(E.rx);
+    if (ntile == 0 || 2 * njobs > 65535) return false;
+    const size_t per_slice = 2 * (size_t)E.nk * sizeof(cx<T>);
+    const int cs = (int)std::max<size_t>(1, std::min<size_t>((size_t)maxs, ((size_t)1 << 30) / (per_slice * njobs)));
+    if (E.spec_bytes < per_slice * cs * njobs) {
+        E.no_growth_in_capture();
+        if (E.spec) cudaFree(E.spec);
+        E.spec = nullptr;
+        E.spec_bytes = 0;
+        CK(cudaMalloc(&E.spec, per_slice * cs * njobs));
+        E.spec_bytes = per_slice * cs * njobs;
+    }
+    const size_t plen = (size_t)cs * njobs * ntile * PSCFG_MAXCP;
+    if (E.stress_part_len < plen) {
+        E.no_growth_in_capture();
+        if (E.stress_part) cudaFree(E.stress_part);
+        E.stress_part = nullptr;
+        E.stress_part_len = 0;
+        CK(cudaMalloc(&E.stress_part, plen * sizeof(double)));
+        E.stress_part_len = plen;
+    }
+    for (int s0 = 0; s0 < maxs; s0 += cs) {
+        const int cnt = std::min(cs, maxs - s0);
+        E.launched_n(rx3_stress<T>(E.rx, E.st, dj, njobs, s0, cnt, cs, (cx<T> *)E.spec, E.stress_part));
+        k3_stress_sum_b<T><<<dim3(cnt, njobs), 32, 0, E.st>>>(dj, s0, cs, ntile, E.stress_part);
+        E.launched();
+    }
+    return true;
+}
+
 template <typename T>
 static void slice_dots(Engine &E, const std::vector<StressJob<T>> &jobs)
 {
@@ -2036,7 +1994,17 @@ static void slice_dots(Engine &E, const std::vector<StressJob<T>> &jobs)
         for (auto &j : jobs) maxs = std::max(maxs, j.nslices);
         if (slice_dots_r<T>(E, dj, (int)jobs.size(), maxs)) return;
     }
+    if (rx3_applies<T>(E)) {
+        int maxs = 0;
+        for (auto &j : jobs) maxs = std::max(maxs, j.nslices);
+        if (slice_dots_v<T>(E, dj, (int)jobs.size(), maxs)) return;
+    }
     size_t off = ((jobs.size() * sizeof(StressJob<T>) + 255) / 256) * 256;
+    if (E.dim == 2 && !E.no_fixed_kernels) {
+        int maxs = 0;
+        for (auto &j : jobs) maxs = std::max(maxs, j.nslices);
+        if (jobs.size() <= 65535 && E.launched_n(rx2_stress<T>(E.rx, E.st, dj, (int)jobs.size(), maxs))) return;
+    }
     if (E.dim <= 2) {
         int maxs = 0;
         for (auto &j : jobs) maxs = std::max(maxs, j.nslices);
@@ -2063,10 +2031,7 @@ static void slice_dots(Engine &E, const std::vector<StressJob<T>> &jobs)
             CK(cudaMalloc(&E.spec, per_slice * cs));
             E.spec_bytes = per_slice * cs;
         }
-        // partial sums per (slice, column tile): the plane kernels' stress
-        // pass (stress3p) tiles by 8 columns, the generic one by Z_TILE
-        const long ntile_max = std::max<long>(ntile, (P + 7) / 8);
-        size_t plen = (size_t)cs * ntile_max * PSCFG_MAXCP;
+        size_t plen = (size_t)cs * ntile * PSCFG_MAXCP;
         if (E.stress_part_len < plen) {
             E.no_growth_in_capture();
             if (E.stress_part) cudaFree(E.stress_part);
@@ -3168,6 +3133,12 @@ static void run_single_steps(Engine &E, const SweepField<T> *dfl, int nf)
 {
     const PlaneGeom &g = E.geom();
     const long nr = E.nr;
+    if (E.dim == 2 && !E.no_fixed_kernels && E.launched_n(rx2_sweep<T>(E.rx, E.st, dfl, nf, 0, 1))) return;
+    if (rx3_applies<T>(E)) {
+        E.launched_n(rx3_first<T>(E.rx, E.st, dfl, nf, 0));
+        E.launched_n(rx3_step<T>(E.rx, E.st, dfl, nf, 0));
+        return;
+    }
     if (E.dim <= 2) {
         size_t sm = 2 * (size_t)g.n2 * g.LS * sizeof(cx<T>) + 2 * (size_t)nr * sizeof(T);
         CK(allow_dyn_smem((const void *)k_sweep_plane<T>));
@@ -4721,6 +4692,7 @@ int pscfg_sweep_planes(const pscfg_engine *e, int n_fields, int fp32)
     if (!e || e->E.dim != 3 || e->E.n[0] != e->E.n[1] || e->E.n[1] != e->E.n[2]) return 0;
     const int n3 = e->E.n[2];
     if (n3 != 16 && n3 != 32) return 0;
+    if (!fp32 && rx3_applies<double>(e->E)) return rx3_planes<double>(e->E.rx, (n_fields + 1) / 2);
     const long key = planes_key(n3, fp32 ? 4 : 8, n_fields);
     std::lock_guard<std::mutex> lk(g_planes_mu);
     auto it = g_planes_best.find(key);

@@ -46,11 +46,6 @@ template <int S, typename T> __device__ __forceinline__ cx<T> mul_si(cx<T> a)
     return (S > 0) ? mk(-a.y, a.x) : mk(a.y, -a.x);
 }
 
-// cos/sin(2 pi m / R) for R = 5 and 7 (m = 0..R-1), filled by the host from
-// long-double evaluations.
-__constant__ double c_dft5[2][5];
-__constant__ double c_dft7[2][7];
-
 // ---------------------------------------------------------------------
 // DFT codelets, in registers.  S = -1 forward, +1 inverse.
 // ---------------------------------------------------------------------
@@ -113,27 +108,29 @@ template <int S, typename T> struct Dft<3, S, T> {
     }
 };
 
-template <int R, int S, typename T> struct DftGeneric {
+// Length-5 DFT from the symmetric pairs t_j = x_j + x_{5-j}, d_j = x_j - x_{5-j}:
+// X_k = x_0 + sum_j cos(2 pi jk/5) t_j + S i sum_j sin(2 pi jk/5) d_j and
+// X_{5-k} the same with -S (k = 1, 2).
+template <int S, typename T> struct Dft<5, S, T> {
     __device__ __forceinline__ static void run(cx<T> *v)
     {
-        const double(*tab)[R] = (R == 5) ? (const double(*)[R])c_dft5 : (const double(*)[R])c_dft7;
-        cx<T> out[R];
-#pragma unroll
-        for (int q = 0; q < R; q++) {
-            cx<T> s = v[0];
-#pragma unroll
-            for (int r = 1; r < R; r++) {
-                int m = (r * q) % R;
-                cx<T> w = mk<T>((T)tab[0][m], (T)S * (T)tab[1][m]);
-                s = s + cmul(v[r], w);
-            }
-            out[q] = s;
-        }
-#pragma unroll
-        for (int q = 0; q < R; q++) v[q] = out[q];
+        const T c1 = (T)0.309016994374947424102293417182819059;    // cos(2 pi/5)
+        const T c2 = (T)-0.809016994374947424102293417182819059;   // cos(4 pi/5)
+        const T s1 = (T)0.951056516295153572116439333379382143;    // sin(2 pi/5)
+        const T s2 = (T)0.587785252292473129168705954639072769;    // sin(4 pi/5)
+        const cx<T> x0 = v[0];
+        const cx<T> t1 = v[1] + v[4], t2 = v[2] + v[3], d1 = v[1] - v[4], d2 = v[2] - v[3];
+        v[0] = x0 + t1 + t2;
+        const cx<T> a1 = mk<T>(x0.x + c1 * t1.x + c2 * t2.x, x0.y + c1 * t1.y + c2 * t2.y);
+        const cx<T> a2 = mk<T>(x0.x + c2 * t1.x + c1 * t2.x, x0.y + c2 * t1.y + c1 * t2.y);
+        const cx<T> b1 = mul_si<S>(mk<T>(s1 * d1.x + s2 * d2.x, s1 * d1.y + s2 * d2.y));
+        const cx<T> b2 = mul_si<S>(mk<T>(s2 * d1.x - s1 * d2.x, s2 * d1.y - s1 * d2.y));
+        v[1] = a1 + b1;
+        v[4] = a1 - b1;
+        v[2] = a2 + b2;
+        v[3] = a2 - b2;
     }
 };
-template <int S, typename T> struct Dft<5, S, T> : DftGeneric<5, S, T> {};
 
 // Length-7 DFT from the symmetric pairs t_j = x_j + x_{7-j}, d_j = x_j - x_{7-j}:
 // X_k = x_0 + sum_j cos(2 pi jk/7) t_j + S i sum_j sin(2 pi jk/7) d_j and

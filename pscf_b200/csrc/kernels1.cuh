@@ -11,6 +11,13 @@
 // the registers of one CTA.  So a CTA forms A once per block (N^3
 // multiply-adds through shared memory) and then walks the contour with one
 // matrix-vector product and one barrier per step.
+//
+// The product is taken about the row's own value,
+//   (A q)_i = (A 1)_i q_i + sum_j A_ij (q_j - q_i),
+// and A 1 from centred circulants, (C x)_i = x_i + sum_j c[i - j] (x_j - x_i)
+// (C 1 = ek(0) = 1): a constant q in a uniform field then stays that constant
+// to the last bit, as it does through exact transforms, and the rounding of
+// A's entries acts on differences only.
 #pragma once
 #include "kernels.cuh"
 
@@ -31,7 +38,7 @@ __global__ void __launch_bounds__(4 * NMAX) k1_sweep_dense(const SweepField<T> *
     constexpr int J = NMAX / 8;
     const SweepField<T> &f = fields[blockIdx.x];
     __shared__ __align__(16) double qs[2][NMAX];
-    __shared__ double c1[2 * NMAX], c2[2 * NMAX], e1[NMAX], e2[NMAX];
+    __shared__ double c1[2 * NMAX], c2[2 * NMAX], e1[NMAX], e2[NMAX], x2[NMAX];
     int blk, src, dst;
     if (!step_slices(f, t0, blk, src, dst)) return;
     const int row = threadIdx.x >> 2, l = threadIdx.x & 3;
@@ -40,7 +47,16 @@ __global__ void __launch_bounds__(4 * NMAX) k1_sweep_dense(const SweepField<T> *
         qs[0][threadIdx.x] = threadIdx.x < n ? (double)q[threadIdx.x] : 0.0;
         qs[1][threadIdx.x] = 0.0;
     }
-    double a[2 * J];
+    // (C x)_row of a shared vector, in all four lanes of the row
+    auto centred = [&](const double *c, const double *x) {
+        const int i = row < n ? row : 0;
+        double s = 0.0;
+        for (int j = l; j < n; j += 4) s += c[i - j + n] * (x[j] - x[i]);
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        return x[i] + s;
+    };
+    double a[2 * J], a1 = 0.0;
     int cur = -1, p = 0;
     for (int t = t0; t < t1; t++) {
         if (!step_slices(f, t, blk, src, dst)) break;
@@ -49,10 +65,11 @@ __global__ void __launch_bounds__(4 * NMAX) k1_sweep_dense(const SweepField<T> *
             __syncthreads();
             // circulants, twice in a row so that c[i - j + n] needs no modulus
             for (int i = threadIdx.x; i < n; i += blockDim.x) {
+                const int d = min(i, n - i);   // c[n - d] = c[d] to the last bit
                 double s1 = 0.0, s2 = 0.0;
                 for (int k = 0; k <= n / 2; k++) {
                     const double w = (k == 0 || 2 * k == n) ? 1.0 : 2.0;
-                    const double c = w * tw[(k * i) % n].x;
+                    const double c = w * tw[(k * d) % n].x;
                     s1 += c * (double)f.ek1[blk][k];
                     s2 += c * (double)f.ek2[blk][k];
                 }
@@ -75,27 +92,32 @@ __global__ void __launch_bounds__(4 * NMAX) k1_sweep_dense(const SweepField<T> *
             }
 #pragma unroll
             for (int j = 0; j < 2 * J; j++) {
-                const int col = min(8 * (j >> 1) + 2 * l + (j & 1), n - 1);
-                a[j] = (4.0 * (e2[i] * a[j] * e2[col]) - e1[i] * c1[i - col + n] * e1[col]) / 3.0;
+                const int cj = 8 * (j >> 1) + 2 * l + (j & 1), col = min(cj, n - 1);
+                a[j] = cj >= n ? 0.0 : (4.0 * (e2[i] * e2[col] * a[j]) - e1[i] * e1[col] * c1[i - col + n]) / 3.0;
             }
+            const double h = e1[i] * centred(c2, e2);
+            if (l == 0 && row < n) x2[row] = h;
+            __syncthreads();
+            a1 = (4.0 * (e2[i] * centred(c2, x2)) - e1[i] * centred(c1, e1)) / 3.0;
         }
         __syncthreads();
         double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+        const double qi = qs[p][row < n ? row : 0];
 #pragma unroll
         for (int j = 0; j < J; j++) {
-            // (columns beyond n meet the zeros kept there)
             const double2 q = *(const double2 *)&qs[p][8 * j + 2 * l];
             if (j & 1) {
-                s2 = fma(a[2 * j], q.x, s2);
-                s3 = fma(a[2 * j + 1], q.y, s3);
+                s2 = fma(a[2 * j], q.x - qi, s2);
+                s3 = fma(a[2 * j + 1], q.y - qi, s3);
             } else {
-                s0 = fma(a[2 * j], q.x, s0);
-                s1 = fma(a[2 * j + 1], q.y, s1);
+                s0 = fma(a[2 * j], q.x - qi, s0);
+                s1 = fma(a[2 * j + 1], q.y - qi, s1);
             }
         }
         double s = (s0 + s1) + (s2 + s3);
         s += __shfl_xor_sync(0xffffffffu, s, 1);
         s += __shfl_xor_sync(0xffffffffu, s, 2);
+        s = fma(a1, qi, s);
         p ^= 1;
         if (l == 0 && row < n) {
             const T v = (T)s;

@@ -72,8 +72,7 @@ static int fail(int code, const std::string &msg)
 // Device address of g_scratch on the current device.  In host code the
 // symbol g_scratch is only a host-side stand-in; the address a kernel may
 // use comes from cudaGetSymbolAddress, looked up once per device (with that
-// device current) on the first call made on it.  The same set-up uploads
-// the radix-5/7 codelet constants of this translation unit.
+// device current) on the first call made on it.
 static int scratch_address(unsigned char **out)
 {
     int dev = 0;
@@ -85,19 +84,6 @@ static int scratch_address(unsigned char **out)
         cudaError_t e = cudaGetSymbolAddress(&p, g_scratch);
         if (e != cudaSuccess || !p)
             return fail(PSCFG_ECUDA, std::string("cudaGetSymbolAddress(g_scratch): ") + cudaGetErrorString(e));
-        double t5[2][5], t7[2][7];
-        for (int m = 0; m < 5; m++) {
-            long double a = 2.0L * 3.14159265358979323846264338327950288L * m / 5.0L;
-            t5[0][m] = (double)cosl(a);
-            t5[1][m] = (double)sinl(a);
-        }
-        for (int m = 0; m < 7; m++) {
-            long double a = 2.0L * 3.14159265358979323846264338327950288L * m / 7.0L;
-            t7[0][m] = (double)cosl(a);
-            t7[1][m] = (double)sinl(a);
-        }
-        CKN(cudaMemcpyToSymbol(c_dft5, t5, sizeof(t5)));
-        CKN(cudaMemcpyToSymbol(c_dft7, t7, sizeof(t7)));
         g_scratch_addr[dev] = (unsigned char *)p;
     }
     *out = g_scratch_addr[dev];

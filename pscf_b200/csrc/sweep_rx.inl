@@ -1,0 +1,218 @@
+// sweep_rx.inl -- launches of the plane_rx.cuh kernels for one type,
+// included by sweep_rx_f64.cu and sweep_rx_f32.cu.
+#include <algorithm>
+
+#include "../../include/pscf_gpu.h"
+#include "launch_util.h"
+#include "sweep_rx.h"
+
+namespace pscfg {
+
+template <typename T> static int prec_of() { return sizeof(T) == 8 ? 0 : 1; }
+
+static const int RX_NT = 288;            // threads of the run-time shaped plane kernels (most)
+static const size_t SMEM_MOST = 226 * 1024;
+static const int RX_SMS = 148;
+
+// threads of a CTA whose largest pass has `items`, in whole rounds
+static int rx_threads(int items, int most = RX_NT)
+{
+    const int rounds = (items + most - 1) / most;
+    const int per = (items + rounds - 1) / rounds;
+    return std::max(32, std::min(most, (per + 31) / 32 * 32));
+}
+
+// planes per CTA: as many as keep the row pass within one round of the
+// threads, fewer where the launch would not fill two CTAs on every SM
+static int rx_ppc(int items, int n3, int nf, size_t plane_bytes)
+{
+    int p = std::max(1, std::min(n3, RX_NT / std::max(items, 1)));
+    while (p > 1 && (p * plane_bytes > 100 * 1024 || (long)nf * ((n3 + p - 1) / p) < 296)) p--;
+    return p;
+}
+
+#define RX_LAUNCH(kernel, grid, block, smem, st, ...)                        \
+    do {                                                                     \
+        if (allow_dyn_smem((const void *)kernel) != cudaSuccess) return -1;  \
+        kernel<<<grid, block, smem, st>>>(__VA_ARGS__);                      \
+        if (cudaPeekAtLastError() != cudaSuccess) return -1;                 \
+    } while (0)
+
+template <typename T, typename SH, int NT, int MB, bool TAB>
+static int sweep2(const RxPlan &p, SH sh, int threads, cudaStream_t st, const SweepField<T> *f, int nf, int t0, int t1)
+{
+    auto *k = k2x_sweep<T, SH, NT, MB, TAB>;
+    RX_LAUNCH(k, nf, threads, rx2_smem<T>(p.sh.n1, p.sh.n2, TAB), st, f, sh, p.tb[prec_of<T>()], t0, t1);
+    return 1;
+}
+
+template <typename T> int rx2_sweep(const RxPlan &p, cudaStream_t st, const SweepField<T> *f, int nf, int t0, int t1)
+{
+    const RxShape &s = p.sh;
+    if (!p.plane || rx2_smem<T>(s.n1, s.n2, false) > SMEM_MOST) return 0;
+    const bool wide = nf <= RX_SMS && rx2_smem<T>(s.n1, s.n2, true) <= SMEM_MOST;
+    if (s.n1 == 64 && s.n2 == 64) {
+        using F = RxFixed<64, 64, 8, 8>;
+        return wide ? sweep2<T, F, 544, 1, true>(p, {}, 544, st, f, nf, t0, t1)
+                    : sweep2<T, F, 288, 2, false>(p, {}, 288, st, f, nf, t0, t1);
+    }
+    const int items = std::max(s.Q2 * s.HP * s.Q1, s.Q2 * s.n1h);
+    return wide ? sweep2<T, RxShape, 544, 1, true>(p, s, rx_threads(std::max(items, 2 * s.P2 * s.n1h), 544), st, f, nf, t0, t1)
+                : sweep2<T, RxShape, RX_NT, 2, false>(p, s, rx_threads(items), st, f, nf, t0, t1);
+}
+
+template <typename T, typename SH, int NT>
+static int stress2(const RxPlan &p, SH sh, int threads, cudaStream_t st, const StressJob<T> *jobs, int njobs, int maxs)
+{
+    auto *k = k2x_stress<T, SH, NT>;
+    RX_LAUNCH(k, dim3(maxs, njobs), threads, rx_smem<T>(p.sh.n1, p.sh.n2, 2 * p.sh.Q2 * p.sh.HP), st, jobs, sh,
+              p.tb[prec_of<T>()]);
+    return 1;
+}
+
+template <typename T> int rx2_stress(const RxPlan &p, cudaStream_t st, const StressJob<T> *jobs, int njobs, int maxs)
+{
+    const RxShape &s = p.sh;
+    if (!p.plane || rx_smem<T>(s.n1, s.n2, 2 * s.Q2 * s.HP) > SMEM_MOST - 1024) return 0;
+    if (s.n1 == 64 && s.n2 == 64) return stress2<T, RxFixed<64, 64, 8, 8>, 288>(p, {}, 288, st, jobs, njobs, maxs);
+    return stress2<T, RxShape, RX_NT>(p, s, rx_threads(std::max(s.Q2 * s.n1h, s.P2 * s.n1h)), st, jobs, njobs, maxs);
+}
+
+// ---------------------------------------------------------------------
+// dim 3
+// ---------------------------------------------------------------------
+template <typename T> static size_t fp_bytes(const RxShape &s, int ppc) { return rx_smem<T>(s.n1, s.n2, ppc * s.n2); }
+template <typename T> static size_t rp_bytes(const RxShape &s, int ppc) { return rx_smem<T>(s.n1, s.n2, ppc * s.Q2 * s.HP); }
+
+template <typename T> bool rx3_fits(const RxPlan &p)
+{
+    return p.plane && p.line && fp_bytes<T>(p.sh, 1) <= SMEM_MOST;
+}
+
+// f(shape, RxInt<threads of FP kernels>, RxInt<their CTAs per SM>, RxInt<threads of k3v_mid>, RxInt<CTAs per SM>)
+template <typename F> static int with_plane(const RxPlan &p, F f)
+{
+    const int a = p.sh.n1, b = p.sh.n2;
+    if (a == 64 && b == 128) return f(RxFixed<64, 128, 8, 8>(), RxInt<544>(), RxInt<1>(), RxInt<288>(), RxInt<2>());
+    if (a == 64 && b == 64) return f(RxFixed<64, 64, 8, 8>(), RxInt<288>(), RxInt<2>(), RxInt<288>(), RxInt<2>());
+    if (a == 32 && b == 32) return f(RxFixed<32, 32, 4, 4>(), RxInt<288>(), RxInt<2>(), RxInt<288>(), RxInt<2>());
+    return f(p.sh, RxInt<RX_NT>(), RxInt<2>(), RxInt<RX_NT>(), RxInt<2>());
+}
+// f(shape, RxInt<columns of a tile>, RxInt<threads>)
+template <typename F> static int with_line(const RxPlan &p, F f)
+{
+    switch (p.z.n3) {
+    case 32: return f(RzFixed<32, 4>(), RxInt<32>(), RxInt<256>());
+    case 64: return f(RzFixed<64, 8>(), RxInt<32>(), RxInt<256>());
+    case 224: return f(RzFixed<224, 16>(), RxInt<16>(), RxInt<256>());
+    default: break;
+    }
+    const int q = std::max(p.z.P, p.z.Q);
+    if (q <= 4) return f(p.z, RxInt<32>(), RxInt<128>());
+    if (q <= 8) return f(p.z, RxInt<32>(), RxInt<256>());
+    return f(p.z, RxInt<16>(), RxInt<256>());
+}
+
+template <typename T> static int fp_threads(const RxShape &s, int ppc, int most)
+{
+    return rx_threads(std::max({ppc * s.n2 * s.Q1, ppc * s.Q2 * s.n1h, ppc * 2 * s.P2 * s.n1h}), most);
+}
+
+template <typename T> int rx3_planes(const RxPlan &p, int nf)
+{
+    return rx_ppc(p.sh.n2 * p.sh.Q1, p.n3, nf, fp_bytes<T>(p.sh, 1));
+}
+
+template <typename T> int rx3_first(const RxPlan &p, cudaStream_t st, const SweepField<T> *f, int nf, int t)
+{
+    if (!rx3_fits<T>(p)) return 0;
+    return with_plane(p, [&](auto sh, auto nt, auto mb, auto, auto) {
+        const int ppc = rx3_planes<T>(p, nf);
+        auto *k = k3v_fwd<T, decltype(sh), decltype(nt)::value, decltype(mb)::value>;
+        RX_LAUNCH(k, dim3((p.n3 + ppc - 1) / ppc, nf), fp_threads<T>(p.sh, ppc, decltype(nt)::value), fp_bytes<T>(p.sh, ppc),
+                  st, f, sh, p.tb[prec_of<T>()], p.n3, ppc, t);
+        return 1;
+    });
+}
+
+template <typename T> static int zconv(const RxPlan &p, cudaStream_t st, const SweepField<T> *f, int nf, int t, int which)
+{
+    return with_line(p, [&](auto z, auto tc, auto nt) {
+        constexpr int TC = decltype(tc)::value, NT = decltype(nt)::value;
+        auto *k = k3v_zconv<T, decltype(z), TC, NT>;
+        RX_LAUNCH(k, dim3((p.sh.n1h * p.sh.n2 + TC - 1) / TC, nf, which == 3 ? 2 : 1), NT, rz_smem<T>(p.n3, TC, 1), st, f, z,
+                  p.zc[prec_of<T>()], t, which);
+        return 1;
+    });
+}
+
+template <typename T> int rx3_step(const RxPlan &p, cudaStream_t st, const SweepField<T> *f, int nf, int t)
+{
+    if (!rx3_fits<T>(p)) return 0;
+    if (zconv<T>(p, st, f, nf, t, 3) < 0) return -1;
+    int rc = with_plane(p, [&](auto sh, auto, auto, auto nt, auto mb) {
+        const RxShape &s = p.sh;
+        const int npair = s.Q2 * s.HP;
+        const int ppc = rx_ppc(npair * s.Q1, p.n3, nf, rp_bytes<T>(s, 1));
+        const int thr = rx_threads(std::max({ppc * npair * s.Q1, ppc * s.Q2 * s.n1h, ppc * s.P2 * s.n1h}), decltype(nt)::value);
+        auto *k = k3v_mid<T, decltype(sh), decltype(nt)::value, decltype(mb)::value>;
+        RX_LAUNCH(k, dim3((p.n3 + ppc - 1) / ppc, nf), thr, rp_bytes<T>(s, ppc), st, f, sh, p.tb[prec_of<T>()], p.n3, ppc, t);
+        return 1;
+    });
+    if (rc < 0 || zconv<T>(p, st, f, nf, t, 2) < 0) return -1;
+    rc = with_plane(p, [&](auto sh, auto nt, auto mb, auto, auto) {
+        const int ppc = rx3_planes<T>(p, nf);
+        auto *k = k3v_final<T, decltype(sh), decltype(nt)::value, decltype(mb)::value>;
+        RX_LAUNCH(k, dim3((p.n3 + ppc - 1) / ppc, nf), fp_threads<T>(p.sh, ppc, decltype(nt)::value), fp_bytes<T>(p.sh, ppc),
+                  st, f, sh, p.tb[prec_of<T>()], p.n3, ppc, t);
+        return 1;
+    });
+    return rc < 0 ? -1 : 4;
+}
+
+// (two tiles of a line have to fit)
+template <typename T> int rx3_stress_tiles(const RxPlan &p)
+{
+    if (!rx3_fits<T>(p)) return 0;
+    return with_line(p, [&](auto, auto tc, auto) {
+        constexpr int TC = decltype(tc)::value;
+        return rz_smem<T>(p.n3, TC, 2) <= SMEM_MOST - 1024 ? (p.sh.n1h * p.sh.n2 + TC - 1) / TC : 0;
+    });
+}
+
+template <typename T>
+int rx3_stress(const RxPlan &p, cudaStream_t st, const StressJob<T> *jobs, int njobs, int s0, int cnt, int cs, cx<T> *spec,
+               double *part)
+{
+    if (rx3_stress_tiles<T>(p) == 0) return 0;
+    const int rc = with_plane(p, [&](auto sh, auto, auto, auto nt, auto mb) {
+        const RxShape &s = p.sh;
+        const int npair = s.Q2 * s.HP;
+        const int ppc = rx_ppc(npair * s.Q1, p.n3, 2 * cnt * njobs, rp_bytes<T>(s, 1));
+        const int thr = rx_threads(std::max({ppc * npair * s.Q1, ppc * s.Q2 * s.n1h, ppc * s.P2 * s.n1h}), decltype(nt)::value);
+        auto *k = k3v_stress_xy<T, decltype(sh), decltype(nt)::value, decltype(mb)::value>;
+        RX_LAUNCH(k, dim3((p.n3 + ppc - 1) / ppc, cnt, 2 * njobs), thr, rp_bytes<T>(s, ppc), st, jobs, sh, p.tb[prec_of<T>()],
+                  p.n3, ppc, s0, cs, spec);
+        return 1;
+    });
+    if (rc < 0) return -1;
+    return with_line(p, [&](auto z, auto tc, auto nt) {
+        constexpr int TC = decltype(tc)::value, NT = decltype(nt)::value;
+        auto *k = k3v_stress_z<T, decltype(z), TC, NT>;
+        RX_LAUNCH(k, dim3((p.sh.n1h * p.sh.n2 + TC - 1) / TC, cnt, njobs), NT, rz_smem<T>(p.n3, TC, 2), st, jobs, z,
+                  p.zc[prec_of<T>()], s0, cs, (const cx<T> *)spec, part);
+        return 2;
+    });
+}
+
+#define RX_INSTANCES(T)                                                                                              \
+    template int rx2_sweep<T>(const RxPlan &, cudaStream_t, const SweepField<T> *, int, int, int);                   \
+    template int rx2_stress<T>(const RxPlan &, cudaStream_t, const StressJob<T> *, int, int);                        \
+    template int rx3_planes<T>(const RxPlan &, int);                                                                 \
+    template bool rx3_fits<T>(const RxPlan &);                                                                       \
+    template int rx3_first<T>(const RxPlan &, cudaStream_t, const SweepField<T> *, int, int);                        \
+    template int rx3_step<T>(const RxPlan &, cudaStream_t, const SweepField<T> *, int, int);                         \
+    template int rx3_stress_tiles<T>(const RxPlan &);                                                                \
+    template int rx3_stress<T>(const RxPlan &, cudaStream_t, const StressJob<T> *, int, int, int, int, cx<T> *, double *);
+
+}  // namespace pscfg
