@@ -189,7 +189,9 @@ template <typename F> __device__ __forceinline__ void rx_q(int r, F f)
     } while (0)
 
 // ---------------------------------------------------------------------
-// Passes.  buf: [line][LS]; tw1, tw2: W_n1^m, W_n2^m in shared memory.
+// Passes.  buf: [line][LS]; in shared memory tw1[Q1 k + r] = W_n1^(r k)
+// (consecutive threads take consecutive r: W_n1^m itself would meet 4-way
+// bank conflicts) and tw2[m] = W_n2^m (one r for a whole warp, mostly).
 // None of them synchronises.
 // ---------------------------------------------------------------------
 template <typename T, typename SH> struct Rx {
@@ -203,7 +205,7 @@ template <typename T, typename SH> struct Rx {
         Dft<P, -1, T>::run(v);
         b[r] = v[0];
 #pragma unroll
-        for (int k = 1; k < P; k++) b[sh.Q1 * k + r] = cmul(v[k], tw1[r * k]);
+        for (int k = 1; k < P; k++) b[sh.Q1 * k + r] = cmul(v[k], tw1[sh.Q1 * k + r]);
     }
     // rows, last pass of the inverse: v[i] = z(Q1 i + r)
     template <int P>
@@ -211,7 +213,7 @@ template <typename T, typename SH> struct Rx {
     {
         v[0] = b[r];
 #pragma unroll
-        for (int k = 1; k < P; k++) v[k] = cmul(b[sh.Q1 * k + r], conjg(tw1[r * k]));
+        for (int k = 1; k < P; k++) v[k] = cmul(b[sh.Q1 * k + r], conjg(tw1[sh.Q1 * k + r]));
         Dft<P, 1, T>::run(v);
     }
     // rows, second forward (S < 0) or first inverse pass of nl lines,
@@ -401,7 +403,10 @@ template <typename T, typename SH> struct RxMem {
         tw1 = buf + lines * sh.LS;
         tw2 = tw1 + sh.n1;
         ct = (RxCol *)(tw2 + sh.n2);
-        for (int i = threadIdx.x; i < sh.n1; i += blockDim.x) tw1[i] = ((const cx<T> *)tb.tw1)[i];
+        for (int i = threadIdx.x; i < sh.n1; i += blockDim.x) {
+            const int k = sh.dQ1.div(i);
+            tw1[i] = ((const cx<T> *)tb.tw1)[k * (i - sh.Q1 * k)];
+        }
         for (int i = threadIdx.x; i < sh.n2; i += blockDim.x) tw2[i] = ((const cx<T> *)tb.tw2)[i];
         for (int i = threadIdx.x; i < sh.n1h; i += blockDim.x) ct[i] = tb.cols[i];
     }
@@ -421,9 +426,13 @@ template <typename T, typename SH> struct RxMem {
 // ---------------------------------------------------------------------
 // TAB: the current block's tables (exp(-w ds/4), and both filters in column
 // order) sit in shared memory too: for launches of at most one CTA per SM.
+// Row stride of its real planes: 8 (mod 16) values, so that the two rows of
+// a half warp lie on different banks.
+__host__ __device__ __forceinline__ constexpr int rx2_stride(int n1) { return n1 + (24 - n1 % 16) % 16; }
 template <typename T> __host__ __device__ constexpr size_t rx2_smem(int n1, int n2, bool tab)
 {
-    return (rx_smem<T>(n1, n2, n2) + 15) / 16 * 16 + sizeof(T) * ((size_t)n1 * n2 * (tab ? 2 : 1) + (tab ? 2 * (n1 / 2 + 1) * n2 : 0));
+    return (rx_smem<T>(n1, n2, n2) + 15) / 16 * 16 +
+           sizeof(T) * ((size_t)rx2_stride(n1) * n2 * (tab ? 2 : 1) + (tab ? 2 * (n1 / 2 + 1) * n2 : 0));
 }
 
 template <typename T, typename SH, int NT, int MB, bool TAB>
@@ -436,7 +445,8 @@ __global__ void __launch_bounds__(NT, MB)
     const RxMem<T, SH> m(sh, tb, sh.n2);
     T *q = (T *)(((size_t)m.end(sh) + 15) / 16 * 16);   // (shared addresses are 16-byte aligned at the buffer)
     const int nr = sh.n1 * sh.n2, nkc = sh.n1h * sh.n2;
-    T *te2 = q + nr, *tek = te2 + nr;   // (TAB)
+    const int QS = rx2_stride(sh.n1);
+    T *te2 = q + QS * sh.n2, *tek = te2 + QS * sh.n2;   // (TAB)
     const T rn = (T)(2.0 * nr), rr = (T)(1.0 / (2.0 * nr)), rt = (T)(1.0 / 3.0);
     const int npair = sh.Q2 * sh.HP;
     const RDiv dpair = RDiv::of(npair), dn2 = RDiv::of(sh.n2);
@@ -444,16 +454,19 @@ __global__ void __launch_bounds__(NT, MB)
     auto row_line = [&](int l) { return l; };
     int blk, src, dst;
     if (!step_slices(f, t0, blk, src, dst)) return;
+    const RDiv dn1 = RDiv::of(sh.n1);
+    auto padded = [&](int i) { const int y = dn1.div(i); return i + (QS - sh.n1) * y; };
     {
         const T *qs = src_slice(f, src, nr);
-        for (int i = threadIdx.x; i < nr; i += blockDim.x) q[i] = qs[i];
+        for (int i = threadIdx.x; i < nr; i += blockDim.x) q[padded(i)] = qs[i];
     }
     __syncthreads();
     // The plane work of one (pair of rows, residue r) item at the row
     // passes' real-space end.  FIRST: q -> FP lines.  MID: FP lines -> q1,
     // h -> RP line.  LAST: RP line -> q_out, then FP lines of the next step.
+    // e2 (with TAB, and e2n if in_table) lies in the padded table.
     enum { FIRST, MID, LAST };
-    auto rows1 = [&](auto phase, const T *e2, const T *e2n, T *out) {
+    auto rows1 = [&](auto phase, const T *e2, const T *e2n, bool in_table, T *out) {
         constexpr int PH = decltype(phase)::value;
         auto go = [&](auto pc) {
             constexpr int P = decltype(pc)::value;
@@ -462,43 +475,46 @@ __global__ void __launch_bounds__(NT, MB)
                 const int y0 = pair_line(l), y1 = y0 + sh.Q2;
                 const bool two = y1 < sh.n2;   // an odd P2 leaves the last row of a residue alone
                 C *b0 = m.buf + y0 * sh.LS, *b1 = m.buf + y1 * sh.LS;
-                const int i0 = y0 * sh.n1 + r, i1 = y1 * sh.n1 + r;
+                const int i0 = y0 * sh.n1 + r, i1 = y1 * sh.n1 + r;   // in global planes
+                const int p0 = y0 * QS + r, p1 = y1 * QS + r;         // in the padded ones
+                const int t0 = TAB ? p0 : i0, t1 = TAB ? p1 : i1;
                 C v[P];
-                T u0[P], u1[P];
+                T u0[P], u1[P], e0[P], e1[P];
+                if (PH != FIRST) {
+                    // (ahead of the stores, which the compiler must assume
+                    // to alias the tables)
+#pragma unroll
+                    for (int i = 0; i < P; i++) {
+                        e0[i] = e2[t0 + sh.Q1 * i];
+                        e1[i] = two ? e2[t1 + sh.Q1 * i] : (T)0;
+                    }
+                }
                 if (PH == FIRST) {
 #pragma unroll
                     for (int i = 0; i < P; i++) {
-                        u0[i] = q[i0 + sh.Q1 * i];
-                        u1[i] = two ? q[i1 + sh.Q1 * i] : (T)0;
+                        u0[i] = q[p0 + sh.Q1 * i];
+                        u1[i] = two ? q[p1 + sh.Q1 * i] : (T)0;
                     }
                 } else if (PH == MID) {
                     // a: first half step, b: full step
-                    T e0[P], e1[P];
-#pragma unroll
-                    for (int i = 0; i < P; i++) {
-                        e0[i] = e2[i0 + sh.Q1 * i];
-                        e1[i] = two ? e2[i1 + sh.Q1 * i] : (T)0;
-                    }
                     X::template row_inv1<P>(sh, b0, r, v, m.tw1);
 #pragma unroll
                     for (int i = 0; i < P; i++) {
-                        const int x = i0 + sh.Q1 * i;
-                        const T ee = e0[i] * e0[i];
-                        q[x] = div_by(ee * v[i].y, rn, rr);
+                        const T ee = e0[i] * e0[i], q1 = div_by(ee * v[i].y, rn, rr);
+                        q[p0 + sh.Q1 * i] = q1;
                         u0[i] = div_by(ee * v[i].x, rn, rr);
-                        if (f.q1) f.q1[x] = q[x];
-                        if (f.h_out) f.h_out[x] = u0[i];
+                        if (f.q1) f.q1[i0 + sh.Q1 * i] = q1;
+                        if (f.h_out) f.h_out[i0 + sh.Q1 * i] = u0[i];
                     }
                     if (two) {
                         X::template row_inv1<P>(sh, b1, r, v, m.tw1);
 #pragma unroll
                         for (int i = 0; i < P; i++) {
-                            const int x = i1 + sh.Q1 * i;
-                            const T ee = e1[i] * e1[i];
-                            q[x] = div_by(ee * v[i].y, rn, rr);
+                            const T ee = e1[i] * e1[i], q1 = div_by(ee * v[i].y, rn, rr);
+                            q[p1 + sh.Q1 * i] = q1;
                             u1[i] = div_by(ee * v[i].x, rn, rr);
-                            if (f.q1) f.q1[x] = q[x];
-                            if (f.h_out) f.h_out[x] = u1[i];
+                            if (f.q1) f.q1[i1 + sh.Q1 * i] = q1;
+                            if (f.h_out) f.h_out[i1 + sh.Q1 * i] = u1[i];
                         }
                     }
 #pragma unroll
@@ -506,41 +522,35 @@ __global__ void __launch_bounds__(NT, MB)
                     X::template row_fwd1<P>(sh, b0, r, v, m.tw1);
                     continue;
                 } else {
-                    T e0[P], e1[P];
-#pragma unroll
-                    for (int i = 0; i < P; i++) {
-                        e0[i] = e2[i0 + sh.Q1 * i];
-                        e1[i] = two ? e2[i1 + sh.Q1 * i] : (T)0;
-                    }
                     X::template row_inv1<P>(sh, b0, r, v, m.tw1);
 #pragma unroll
                     for (int i = 0; i < P; i++) {
-                        const int x = i0 + sh.Q1 * i, y = i1 + sh.Q1 * i;
                         const T qa = div_by(e0[i] * v[i].x, rn, rr);
-                        u0[i] = div_by((T)4 * qa - q[x], (T)3, rt);
-                        q[x] = u0[i];
-                        out[x] = u0[i];
-                        if (f.q2_out) f.q2_out[x] = qa;
+                        u0[i] = div_by((T)4 * qa - q[p0 + sh.Q1 * i], (T)3, rt);
+                        q[p0 + sh.Q1 * i] = u0[i];
+                        out[i0 + sh.Q1 * i] = u0[i];
+                        if (f.q2_out) f.q2_out[i0 + sh.Q1 * i] = qa;
                         if (two) {
                             const T qb = div_by(e1[i] * v[i].y, rn, rr);
-                            u1[i] = div_by((T)4 * qb - q[y], (T)3, rt);
-                            q[y] = u1[i];
-                            out[y] = u1[i];
-                            if (f.q2_out) f.q2_out[y] = qb;
+                            u1[i] = div_by((T)4 * qb - q[p1 + sh.Q1 * i], (T)3, rt);
+                            q[p1 + sh.Q1 * i] = u1[i];
+                            out[i1 + sh.Q1 * i] = u1[i];
+                            if (f.q2_out) f.q2_out[i1 + sh.Q1 * i] = qb;
                         }
                     }
                     if (!e2n) continue;
                 }
+                const int n0 = in_table ? p0 : i0, n1 = in_table ? p1 : i1;
 #pragma unroll
                 for (int i = 0; i < P; i++) {
-                    const T e = e2n[i0 + sh.Q1 * i], a = e * u0[i];
+                    const T e = e2n[n0 + sh.Q1 * i], a = e * u0[i];
                     v[i] = mk<T>(a, e * a);
                 }
                 X::template row_fwd1<P>(sh, b0, r, v, m.tw1);
                 if (two) {
 #pragma unroll
                     for (int i = 0; i < P; i++) {
-                        const T e = e2n[i1 + sh.Q1 * i], a = e * u1[i];
+                        const T e = e2n[n1 + sh.Q1 * i], a = e * u1[i];
                         v[i] = mk<T>(a, e * a);
                     }
                     X::template row_fwd1<P>(sh, b1, r, v, m.tw1);
@@ -580,14 +590,14 @@ __global__ void __launch_bounds__(NT, MB)
         else X::template rows2<1>(sh, m.buf, npair, dpair, pair_line);
         __syncthreads();
     };
-    rows1(RxInt<FIRST>(), nullptr, f.eo2[blk], nullptr);
+    rows1(RxInt<FIRST>(), nullptr, f.eo2[blk], false, nullptr);
     int cur = -1;
     for (int t = t0; t < t1; t++) {
         if (!step_slices(f, t, blk, src, dst)) break;
         if (TAB && blk != cur) {
             cur = blk;
             __syncthreads();
-            for (int i = threadIdx.x; i < nr; i += blockDim.x) te2[i] = f.eo2[blk][i];
+            for (int i = threadIdx.x; i < nr; i += blockDim.x) te2[padded(i)] = f.eo2[blk][i];
             for (int i = threadIdx.x; i < nkc; i += blockDim.x) {
                 const int ky = sh.dn1h.div(i), k = m.ct[i - sh.n1h * ky].kx + sh.n1h * ky;
                 tek[i] = f.ek2[blk][k];
@@ -596,11 +606,11 @@ __global__ void __launch_bounds__(NT, MB)
         }
         const T *e2 = TAB ? te2 : f.eo2[blk], *k2 = TAB ? tek : f.ek2[blk], *k1 = TAB ? tek + nkc : f.ek1[blk];
         conv(RxInt<1>(), k2, k1);
-        rows1(RxInt<MID>(), e2, nullptr, nullptr);
+        rows1(RxInt<MID>(), e2, nullptr, false, nullptr);
         conv(RxInt<0>(), k2, nullptr);
         int blk2, src2, dst2;
         const bool next = t + 1 < t1 && step_slices(f, t + 1, blk2, src2, dst2);
-        rows1(RxInt<LAST>(), e2, !next ? nullptr : blk2 == blk ? e2 : f.eo2[blk2], dst_slice(f, dst, nr));
+        rows1(RxInt<LAST>(), e2, !next ? nullptr : blk2 == blk ? e2 : f.eo2[blk2], TAB && next && blk2 == blk, dst_slice(f, dst, nr));
     }
 }
 

@@ -90,9 +90,14 @@ template <typename T> bool rx3_fits(const RxPlan &p)
 }
 
 // f(shape, RxInt<threads of FP kernels>, RxInt<their CTAs per SM>, RxInt<threads of k3v_mid>, RxInt<CTAs per SM>)
-template <typename F> static int with_plane(const RxPlan &p, F f)
+// for launches of `ctas` CTAs: with at most one per SM each gets twice the threads
+template <typename F> static int with_plane(const RxPlan &p, int ctas, F f)
 {
     const int a = p.sh.n1, b = p.sh.n2;
+    if (ctas <= RX_SMS) {
+        if (a == 64 && b == 64) return f(RxFixed<64, 64, 8, 8>(), RxInt<544>(), RxInt<1>(), RxInt<288>(), RxInt<2>());
+        if (!(a == 64 && b == 128) && !(a == 32 && b == 32)) return f(p.sh, RxInt<544>(), RxInt<1>(), RxInt<RX_NT>(), RxInt<2>());
+    }
     if (a == 64 && b == 128) return f(RxFixed<64, 128, 8, 8>(), RxInt<544>(), RxInt<1>(), RxInt<288>(), RxInt<2>());
     if (a == 64 && b == 64) return f(RxFixed<64, 64, 8, 8>(), RxInt<288>(), RxInt<2>(), RxInt<288>(), RxInt<2>());
     if (a == 32 && b == 32) return f(RxFixed<32, 32, 4, 4>(), RxInt<288>(), RxInt<2>(), RxInt<288>(), RxInt<2>());
@@ -123,10 +128,16 @@ template <typename T> int rx3_planes(const RxPlan &p, int nf)
     return rx_ppc(p.sh.n2 * p.sh.Q1, p.n3, nf, fp_bytes<T>(p.sh, 1));
 }
 
+template <typename T> static int rx3_ctas(const RxPlan &p, int nf)
+{
+    const int ppc = rx3_planes<T>(p, nf);
+    return (p.n3 + ppc - 1) / ppc * nf;
+}
+
 template <typename T> int rx3_first(const RxPlan &p, cudaStream_t st, const SweepField<T> *f, int nf, int t)
 {
     if (!rx3_fits<T>(p)) return 0;
-    return with_plane(p, [&](auto sh, auto nt, auto mb, auto, auto) {
+    return with_plane(p, rx3_ctas<T>(p, nf), [&](auto sh, auto nt, auto mb, auto, auto) {
         const int ppc = rx3_planes<T>(p, nf);
         auto *k = k3v_fwd<T, decltype(sh), decltype(nt)::value, decltype(mb)::value>;
         RX_LAUNCH(k, dim3((p.n3 + ppc - 1) / ppc, nf), fp_threads<T>(p.sh, ppc, decltype(nt)::value), fp_bytes<T>(p.sh, ppc),
@@ -150,7 +161,7 @@ template <typename T> int rx3_step(const RxPlan &p, cudaStream_t st, const Sweep
 {
     if (!rx3_fits<T>(p)) return 0;
     if (zconv<T>(p, st, f, nf, t, 3) < 0) return -1;
-    int rc = with_plane(p, [&](auto sh, auto, auto, auto nt, auto mb) {
+    int rc = with_plane(p, 1 << 30, [&](auto sh, auto, auto, auto nt, auto mb) {
         const RxShape &s = p.sh;
         const int npair = s.Q2 * s.HP;
         const int ppc = rx_ppc(npair * s.Q1, p.n3, nf, rp_bytes<T>(s, 1));
@@ -160,7 +171,7 @@ template <typename T> int rx3_step(const RxPlan &p, cudaStream_t st, const Sweep
         return 1;
     });
     if (rc < 0 || zconv<T>(p, st, f, nf, t, 2) < 0) return -1;
-    rc = with_plane(p, [&](auto sh, auto nt, auto mb, auto, auto) {
+    rc = with_plane(p, rx3_ctas<T>(p, nf), [&](auto sh, auto nt, auto mb, auto, auto) {
         const int ppc = rx3_planes<T>(p, nf);
         auto *k = k3v_final<T, decltype(sh), decltype(nt)::value, decltype(mb)::value>;
         RX_LAUNCH(k, dim3((p.n3 + ppc - 1) / ppc, nf), fp_threads<T>(p.sh, ppc, decltype(nt)::value), fp_bytes<T>(p.sh, ppc),
@@ -185,7 +196,7 @@ int rx3_stress(const RxPlan &p, cudaStream_t st, const StressJob<T> *jobs, int n
                double *part)
 {
     if (rx3_stress_tiles<T>(p) == 0) return 0;
-    const int rc = with_plane(p, [&](auto sh, auto, auto, auto nt, auto mb) {
+    const int rc = with_plane(p, 1 << 30, [&](auto sh, auto, auto, auto nt, auto mb) {
         const RxShape &s = p.sh;
         const int npair = s.Q2 * s.HP;
         const int ppc = rx_ppc(npair * s.Q1, p.n3, 2 * cnt * njobs, rp_bytes<T>(s, 1));
