@@ -130,11 +130,17 @@ __host__ __device__ __forceinline__ constexpr int rx_slot(int Q1, int k1, int k2
 // line stride in complex values: n1 slots, two spare ones, odd
 __host__ __device__ __forceinline__ constexpr int rx_stride(int n1) { return (n1 + 2) | 1; }
 
-// run-time plane shape
+// run-time plane shape; PM, QM: the largest radices a kernel is compiled for
+// (a kernel takes the registers of its largest radix; lines up to 64 points
+// do with 8 and 10)
 struct RxShape {
     static constexpr bool FIXED = false;
+    static constexpr int PM = 10, QM = 16;
     int n1, n2, n1h, P1, Q1, P2, Q2, HP, LS;
     RDiv dQ1, dn1h, dQ2, dP2, dn2;
+};
+struct RxShape10 : RxShape {
+    static constexpr int PM = 8, QM = 10;
 };
 // compile-time plane shape
 template <int N1, int N2, int P1_, int P2_> struct RxFixed {
@@ -153,8 +159,12 @@ template <int V> struct RxInt {
 };
 // f(RxInt<radix>) for the first radix of a line (1..10, rows also 12..16
 // through rx_q) or the second
-template <typename F> __device__ __forceinline__ void rx_p(int r, F f)
+template <int PM, typename F> __device__ __forceinline__ void rx_p(int r, F f)
 {
+    if constexpr (PM > 8) {
+        if (r == 9) return f(RxInt<9>());
+        if (r == 10) return f(RxInt<10>());
+    }
     switch (r) {
     case 1: f(RxInt<1>()); break;
     case 2: f(RxInt<2>()); break;
@@ -164,28 +174,29 @@ template <typename F> __device__ __forceinline__ void rx_p(int r, F f)
     case 6: f(RxInt<6>()); break;
     case 7: f(RxInt<7>()); break;
     case 8: f(RxInt<8>()); break;
-    case 9: f(RxInt<9>()); break;
-    case 10: f(RxInt<10>()); break;
     default: break;
     }
 }
-template <typename F> __device__ __forceinline__ void rx_q(int r, F f)
+template <int QM, typename F> __device__ __forceinline__ void rx_q(int r, F f)
 {
-    switch (r) {
-    case 12: f(RxInt<12>()); break;
-    case 14: f(RxInt<14>()); break;
-    case 15: f(RxInt<15>()); break;
-    case 16: f(RxInt<16>()); break;
-    default: rx_p(r, f); break;
+    if constexpr (QM > 10) {
+        switch (r) {
+        case 12: f(RxInt<12>()); return;
+        case 14: f(RxInt<14>()); return;
+        case 15: f(RxInt<15>()); return;
+        case 16: f(RxInt<16>()); return;
+        default: break;
+        }
     }
+    rx_p<10>(r, f);
 }
 #define RX_P(SH, r, F)                                             \
     do {                                                           \
-        if constexpr (SH::FIXED) F(RxInt<SH::r>()); else rx_p(sh.r, F); \
+        if constexpr (SH::FIXED) F(RxInt<SH::r>()); else rx_p<SH::PM>(sh.r, F); \
     } while (0)
 #define RX_Q(SH, r, F)                                             \
     do {                                                           \
-        if constexpr (SH::FIXED) F(RxInt<SH::r>()); else rx_q(sh.r, F); \
+        if constexpr (SH::FIXED) F(RxInt<SH::r>()); else rx_q<SH::QM>(sh.r, F); \
     } while (0)
 
 // ---------------------------------------------------------------------
@@ -479,16 +490,13 @@ __global__ void __launch_bounds__(NT, MB)
                 const int p0 = y0 * QS + r, p1 = y1 * QS + r;         // in the padded ones
                 const int t0 = TAB ? p0 : i0, t1 = TAB ? p1 : i1;
                 C v[P];
-                T u0[P], u1[P], e0[P], e1[P];
-                if (PH != FIRST) {
-                    // (ahead of the stores, which the compiler must assume
-                    // to alias the tables)
+                T u0[P], u1[P], e[P];
+                // (a row's table values ahead of its stores, which the
+                // compiler must assume to alias the tables)
+                auto load_e = [&](const T *src) {
 #pragma unroll
-                    for (int i = 0; i < P; i++) {
-                        e0[i] = e2[t0 + sh.Q1 * i];
-                        e1[i] = two ? e2[t1 + sh.Q1 * i] : (T)0;
-                    }
-                }
+                    for (int i = 0; i < P; i++) e[i] = src[sh.Q1 * i];
+                };
                 if (PH == FIRST) {
 #pragma unroll
                     for (int i = 0; i < P; i++) {
@@ -497,20 +505,22 @@ __global__ void __launch_bounds__(NT, MB)
                     }
                 } else if (PH == MID) {
                     // a: first half step, b: full step
+                    load_e(e2 + t0);
                     X::template row_inv1<P>(sh, b0, r, v, m.tw1);
 #pragma unroll
                     for (int i = 0; i < P; i++) {
-                        const T ee = e0[i] * e0[i], q1 = div_by(ee * v[i].y, rn, rr);
+                        const T ee = e[i] * e[i], q1 = div_by(ee * v[i].y, rn, rr);
                         q[p0 + sh.Q1 * i] = q1;
                         u0[i] = div_by(ee * v[i].x, rn, rr);
                         if (f.q1) f.q1[i0 + sh.Q1 * i] = q1;
                         if (f.h_out) f.h_out[i0 + sh.Q1 * i] = u0[i];
                     }
                     if (two) {
+                        load_e(e2 + t1);
                         X::template row_inv1<P>(sh, b1, r, v, m.tw1);
 #pragma unroll
                         for (int i = 0; i < P; i++) {
-                            const T ee = e1[i] * e1[i], q1 = div_by(ee * v[i].y, rn, rr);
+                            const T ee = e[i] * e[i], q1 = div_by(ee * v[i].y, rn, rr);
                             q[p1 + sh.Q1 * i] = q1;
                             u1[i] = div_by(ee * v[i].x, rn, rr);
                             if (f.q1) f.q1[i1 + sh.Q1 * i] = q1;
@@ -522,21 +532,22 @@ __global__ void __launch_bounds__(NT, MB)
                     X::template row_fwd1<P>(sh, b0, r, v, m.tw1);
                     continue;
                 } else {
+                    load_e(e2 + t0);
                     X::template row_inv1<P>(sh, b0, r, v, m.tw1);
+                    auto row = [&](T *u, int pr, int ir, bool second) {
 #pragma unroll
-                    for (int i = 0; i < P; i++) {
-                        const T qa = div_by(e0[i] * v[i].x, rn, rr);
-                        u0[i] = div_by((T)4 * qa - q[p0 + sh.Q1 * i], (T)3, rt);
-                        q[p0 + sh.Q1 * i] = u0[i];
-                        out[i0 + sh.Q1 * i] = u0[i];
-                        if (f.q2_out) f.q2_out[i0 + sh.Q1 * i] = qa;
-                        if (two) {
-                            const T qb = div_by(e1[i] * v[i].y, rn, rr);
-                            u1[i] = div_by((T)4 * qb - q[p1 + sh.Q1 * i], (T)3, rt);
-                            q[p1 + sh.Q1 * i] = u1[i];
-                            out[i1 + sh.Q1 * i] = u1[i];
-                            if (f.q2_out) f.q2_out[i1 + sh.Q1 * i] = qb;
+                        for (int i = 0; i < P; i++) {
+                            const T q2 = div_by(e[i] * (second ? v[i].y : v[i].x), rn, rr);
+                            u[i] = div_by((T)4 * q2 - q[pr + sh.Q1 * i], (T)3, rt);
+                            q[pr + sh.Q1 * i] = u[i];
+                            out[ir + sh.Q1 * i] = u[i];
+                            if (f.q2_out) f.q2_out[ir + sh.Q1 * i] = q2;
                         }
+                    };
+                    row(u0, p0, i0, false);
+                    if (two) {
+                        load_e(e2 + t1);
+                        row(u1, p1, i1, true);
                     }
                     if (!e2n) continue;
                 }
@@ -956,7 +967,11 @@ __global__ void __launch_bounds__(NT, MB)
 // ---------------------------------------------------------------------
 struct RzShape {
     static constexpr bool FIXED = false;
+    static constexpr int QM = 16;
     int n3, P, Q;
+};
+struct RzShape10 : RzShape {
+    static constexpr int QM = 10;
 };
 template <int N3, int P_> struct RzFixed {
     static constexpr bool FIXED = true;
@@ -975,8 +990,8 @@ struct RzCols {
 // grid = (ceil(n1h n2 / TC), nfields, 1 or 2); which: 1 = S1/ek1, 2 =
 // S2/ek2, 3 = both (grid.z selects).  ekf: the filter as products of 1-D
 // factors over kx, ky, kz (orthogonal cells), which saves the read of ek.
-template <typename T, typename ZS, int TC, int NT>
-__global__ void __launch_bounds__(NT, 512 / NT) k3v_zconv(const SweepField<T> *fields, ZS sh, RzCols g, int t, int which)
+template <typename T, typename ZS, int TC, int NT, int MB>
+__global__ void __launch_bounds__(NT, MB) k3v_zconv(const SweepField<T> *fields, ZS sh, RzCols g, int t, int which)
 {
     using C = cx<T>;
     const SweepField<T> &f = fields[blockIdx.y];

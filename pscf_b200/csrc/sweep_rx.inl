@@ -14,6 +14,8 @@ static const int RX_NT = 288;            // threads of the run-time shaped plane
 static const size_t SMEM_MOST = 226 * 1024;
 static const int RX_SMS = 148;
 
+static bool small10(const RxShape &s) { return s.P1 <= 8 && s.Q1 <= 10 && s.P2 <= 8 && s.Q2 <= 10; }
+
 // threads of a CTA whose largest pass has `items`, in whole rounds
 static int rx_threads(int items, int most = RX_NT)
 {
@@ -57,8 +59,12 @@ template <typename T> int rx2_sweep(const RxPlan &p, cudaStream_t st, const Swee
                     : sweep2<T, F, 288, 2, false>(p, {}, 288, st, f, nf, t0, t1);
     }
     const int items = std::max(s.Q2 * s.HP * s.Q1, s.Q2 * s.n1h);
-    return wide ? sweep2<T, RxShape, 544, 1, true>(p, s, rx_threads(std::max(items, 2 * s.P2 * s.n1h), 544), st, f, nf, t0, t1)
-                : sweep2<T, RxShape, RX_NT, 2, false>(p, s, rx_threads(items), st, f, nf, t0, t1);
+    auto go = [&](auto sh) {
+        using SH = decltype(sh);
+        return wide ? sweep2<T, SH, 544, 1, true>(p, sh, rx_threads(std::max(items, 2 * s.P2 * s.n1h), 544), st, f, nf, t0, t1)
+                    : sweep2<T, SH, RX_NT, 2, false>(p, sh, rx_threads(items), st, f, nf, t0, t1);
+    };
+    return small10(s) ? go(RxShape10{s}) : go(s);
 }
 
 template <typename T, typename SH, int NT>
@@ -90,32 +96,48 @@ template <typename T> bool rx3_fits(const RxPlan &p)
 }
 
 // f(shape, RxInt<threads of FP kernels>, RxInt<their CTAs per SM>, RxInt<threads of k3v_mid>, RxInt<CTAs per SM>)
-// for launches of `ctas` CTAs: with at most one per SM each gets twice the threads
-template <typename F> static int with_plane(const RxPlan &p, int ctas, F f)
+// for launches of `ctas` CTAs: with at most one per SM each gets twice the
+// threads.  FP32 values take half the registers: more CTAs per SM.
+template <typename T, typename F> static int with_plane(const RxPlan &p, int ctas, F f)
 {
+    constexpr bool F32 = sizeof(T) == 4;
     const int a = p.sh.n1, b = p.sh.n2;
-    if (ctas <= RX_SMS) {
-        if (a == 64 && b == 64) return f(RxFixed<64, 64, 8, 8>(), RxInt<544>(), RxInt<1>(), RxInt<288>(), RxInt<2>());
-        if (!(a == 64 && b == 128) && !(a == 32 && b == 32)) return f(p.sh, RxInt<544>(), RxInt<1>(), RxInt<RX_NT>(), RxInt<2>());
+    if (a == 64 && b == 128)
+        return f(RxFixed<64, 128, 8, 8>(), RxInt<F32 ? 288 : 544>(), RxInt<F32 ? 3 : 1>(), RxInt<288>(), RxInt<F32 ? 4 : 2>());
+    if (a == 32 && b == 32) return f(RxFixed<32, 32, 4, 4>(), RxInt<288>(), RxInt<3>(), RxInt<288>(), RxInt<3>());
+    if (a == 64 && b == 64) {
+        using S = RxFixed<64, 64, 8, 8>;
+        if (ctas <= RX_SMS) return f(S(), RxInt<544>(), RxInt<1>(), RxInt<288>(), RxInt<2>());
+        return f(S(), RxInt<288>(), RxInt<F32 ? 3 : 2>(), RxInt<288>(), RxInt<F32 ? 4 : 2>());
     }
-    if (a == 64 && b == 128) return f(RxFixed<64, 128, 8, 8>(), RxInt<544>(), RxInt<1>(), RxInt<288>(), RxInt<2>());
-    if (a == 64 && b == 64) return f(RxFixed<64, 64, 8, 8>(), RxInt<288>(), RxInt<2>(), RxInt<288>(), RxInt<2>());
-    if (a == 32 && b == 32) return f(RxFixed<32, 32, 4, 4>(), RxInt<288>(), RxInt<2>(), RxInt<288>(), RxInt<2>());
-    return f(p.sh, RxInt<RX_NT>(), RxInt<2>(), RxInt<RX_NT>(), RxInt<2>());
+    auto go = [&](auto sh) {
+        if (ctas <= RX_SMS) return f(sh, RxInt<544>(), RxInt<1>(), RxInt<RX_NT>(), RxInt<2>());
+        return f(sh, RxInt<RX_NT>(), RxInt<2>(), RxInt<RX_NT>(), RxInt<2>());
+    };
+    return small10(p.sh) ? go(RxShape10{p.sh}) : go(p.sh);
 }
-// f(shape, RxInt<columns of a tile>, RxInt<threads>)
-template <typename F> static int with_line(const RxPlan &p, F f)
+// f(shape, RxInt<columns of a tile>, RxInt<threads>, RxInt<CTAs per SM of the
+// filter pass>), for nf spectra: half as wide where the wide tiles would
+// leave SMs idle
+template <typename T, typename F> static int with_line(const RxPlan &p, int nf, F f)
 {
+    constexpr bool F32 = sizeof(T) == 4;
+    const bool narrow = (long)p.sh.n1h * p.sh.n2 * nf < 32L * 2 * RX_SMS;
     switch (p.z.n3) {
-    case 32: return f(RzFixed<32, 4>(), RxInt<32>(), RxInt<256>());
-    case 64: return f(RzFixed<64, 8>(), RxInt<32>(), RxInt<256>());
-    case 224: return f(RzFixed<224, 16>(), RxInt<16>(), RxInt<256>());
+    case 32:
+        if (narrow) return f(RzFixed<32, 8>(), RxInt<8>(), RxInt<64>(), RxInt<8>());
+        return f(RzFixed<32, 8>(), RxInt<32>(), RxInt<256>(), RxInt<4>());
+    case 64:
+        if (narrow) return f(RzFixed<64, 8>(), RxInt<16>(), RxInt<128>(), RxInt<4>());
+        return f(RzFixed<64, 8>(), RxInt<32>(), RxInt<256>(), RxInt<F32 ? 4 : 2>());
+    case 224: return f(RzFixed<224, 16>(), RxInt<16>(), RxInt<256>(), RxInt<F32 ? 3 : 2>());
     default: break;
     }
     const int q = std::max(p.z.P, p.z.Q);
-    if (q <= 4) return f(p.z, RxInt<32>(), RxInt<128>());
-    if (q <= 8) return f(p.z, RxInt<32>(), RxInt<256>());
-    return f(p.z, RxInt<16>(), RxInt<256>());
+    if (q <= 8 && narrow) return f(RzShape10{p.z}, RxInt<16>(), RxInt<128>(), RxInt<4>());
+    if (q <= 8) return f(RzShape10{p.z}, RxInt<32>(), RxInt<256>(), RxInt<3>());
+    if (q <= 10) return f(RzShape10{p.z}, RxInt<16>(), RxInt<160>(), RxInt<4>());
+    return f(p.z, RxInt<16>(), RxInt<256>(), RxInt<2>());
 }
 
 template <typename T> static int fp_threads(const RxShape &s, int ppc, int most)
@@ -137,7 +159,7 @@ template <typename T> static int rx3_ctas(const RxPlan &p, int nf)
 template <typename T> int rx3_first(const RxPlan &p, cudaStream_t st, const SweepField<T> *f, int nf, int t)
 {
     if (!rx3_fits<T>(p)) return 0;
-    return with_plane(p, rx3_ctas<T>(p, nf), [&](auto sh, auto nt, auto mb, auto, auto) {
+    return with_plane<T>(p, rx3_ctas<T>(p, nf), [&](auto sh, auto nt, auto mb, auto, auto) {
         const int ppc = rx3_planes<T>(p, nf);
         auto *k = k3v_fwd<T, decltype(sh), decltype(nt)::value, decltype(mb)::value>;
         RX_LAUNCH(k, dim3((p.n3 + ppc - 1) / ppc, nf), fp_threads<T>(p.sh, ppc, decltype(nt)::value), fp_bytes<T>(p.sh, ppc),
@@ -148,9 +170,9 @@ template <typename T> int rx3_first(const RxPlan &p, cudaStream_t st, const Swee
 
 template <typename T> static int zconv(const RxPlan &p, cudaStream_t st, const SweepField<T> *f, int nf, int t, int which)
 {
-    return with_line(p, [&](auto z, auto tc, auto nt) {
+    return with_line<T>(p, nf * (which == 3 ? 2 : 1), [&](auto z, auto tc, auto nt, auto mb) {
         constexpr int TC = decltype(tc)::value, NT = decltype(nt)::value;
-        auto *k = k3v_zconv<T, decltype(z), TC, NT>;
+        auto *k = k3v_zconv<T, decltype(z), TC, NT, decltype(mb)::value>;
         RX_LAUNCH(k, dim3((p.sh.n1h * p.sh.n2 + TC - 1) / TC, nf, which == 3 ? 2 : 1), NT, rz_smem<T>(p.n3, TC, 1), st, f, z,
                   p.zc[prec_of<T>()], t, which);
         return 1;
@@ -161,7 +183,7 @@ template <typename T> int rx3_step(const RxPlan &p, cudaStream_t st, const Sweep
 {
     if (!rx3_fits<T>(p)) return 0;
     if (zconv<T>(p, st, f, nf, t, 3) < 0) return -1;
-    int rc = with_plane(p, 1 << 30, [&](auto sh, auto, auto, auto nt, auto mb) {
+    int rc = with_plane<T>(p, 1 << 30, [&](auto sh, auto, auto, auto nt, auto mb) {
         const RxShape &s = p.sh;
         const int npair = s.Q2 * s.HP;
         const int ppc = rx_ppc(npair * s.Q1, p.n3, nf, rp_bytes<T>(s, 1));
@@ -171,7 +193,7 @@ template <typename T> int rx3_step(const RxPlan &p, cudaStream_t st, const Sweep
         return 1;
     });
     if (rc < 0 || zconv<T>(p, st, f, nf, t, 2) < 0) return -1;
-    rc = with_plane(p, rx3_ctas<T>(p, nf), [&](auto sh, auto nt, auto mb, auto, auto) {
+    rc = with_plane<T>(p, rx3_ctas<T>(p, nf), [&](auto sh, auto nt, auto mb, auto, auto) {
         const int ppc = rx3_planes<T>(p, nf);
         auto *k = k3v_final<T, decltype(sh), decltype(nt)::value, decltype(mb)::value>;
         RX_LAUNCH(k, dim3((p.n3 + ppc - 1) / ppc, nf), fp_threads<T>(p.sh, ppc, decltype(nt)::value), fp_bytes<T>(p.sh, ppc),
@@ -185,7 +207,7 @@ template <typename T> int rx3_step(const RxPlan &p, cudaStream_t st, const Sweep
 template <typename T> int rx3_stress_tiles(const RxPlan &p)
 {
     if (!rx3_fits<T>(p)) return 0;
-    return with_line(p, [&](auto, auto tc, auto) {
+    return with_line<T>(p, 1 << 20, [&](auto, auto tc, auto, auto) {
         constexpr int TC = decltype(tc)::value;
         return rz_smem<T>(p.n3, TC, 2) <= SMEM_MOST - 1024 ? (p.sh.n1h * p.sh.n2 + TC - 1) / TC : 0;
     });
@@ -196,7 +218,7 @@ int rx3_stress(const RxPlan &p, cudaStream_t st, const StressJob<T> *jobs, int n
                double *part)
 {
     if (rx3_stress_tiles<T>(p) == 0) return 0;
-    const int rc = with_plane(p, 1 << 30, [&](auto sh, auto, auto, auto nt, auto mb) {
+    const int rc = with_plane<T>(p, 1 << 30, [&](auto sh, auto, auto, auto nt, auto mb) {
         const RxShape &s = p.sh;
         const int npair = s.Q2 * s.HP;
         const int ppc = rx_ppc(npair * s.Q1, p.n3, 2 * cnt * njobs, rp_bytes<T>(s, 1));
@@ -207,7 +229,7 @@ int rx3_stress(const RxPlan &p, cudaStream_t st, const StressJob<T> *jobs, int n
         return 1;
     });
     if (rc < 0) return -1;
-    return with_line(p, [&](auto z, auto tc, auto nt) {
+    return with_line<T>(p, 1 << 20, [&](auto z, auto tc, auto nt, auto) {
         constexpr int TC = decltype(tc)::value, NT = decltype(nt)::value;
         auto *k = k3v_stress_z<T, decltype(z), TC, NT>;
         RX_LAUNCH(k, dim3((p.sh.n1h * p.sh.n2 + TC - 1) / TC, cnt, njobs), NT, rz_smem<T>(p.n3, TC, 2), st, jobs, z,

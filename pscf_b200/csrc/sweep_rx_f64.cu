@@ -7,14 +7,15 @@ static bool has_radix(int r, bool first) { return (r >= 1 && r <= 10) || (!first
 
 // N = P Q with the least P + Q; rows and z lines want the wider second
 // factor (consecutive threads load Q consecutive points), columns an even P
-// (rows go in pairs of one residue class).
+// (rows go in pairs of one residue class); first factors above 8 only where
+// there is no other.
 static bool split(int n, bool first_small, bool even, int &P, int &Q)
 {
     int best = 1 << 30;
     for (int p = 1; p <= 16; p++) {
         if (n % p || !has_radix(p, first_small) || !has_radix(n / p, false)) continue;
         const int q = n / p;
-        const int cost = 4 * (p + q) + (even && (p & 1) && p > 1 ? 8 : 0) + (!even && q < p ? 1 : 0);
+        const int cost = 4 * (p + q) + (even && (p & 1) && p > 1 ? 8 : 0) + (!even && q < p ? 1 : 0) + (first_small && p > 8 ? 100 : 0);
         if (cost < best) {
             best = cost;
             P = p;
@@ -54,7 +55,7 @@ bool rx_shape(int dim, const int n[3], RxPlan &p, RxCol *cols)
         for (int kx = k1; 2 * kx < s.n1; kx += s.P1) add(kx);
     if (s.n1 % 2 == 0) add(s.n1 / 2);
     p.z.n3 = p.n3;
-    p.line = dim == 3 && split(p.n3, false, false, p.z.P, p.z.Q);
+    p.line = dim == 3 && split(p.n3, false, false, p.z.Q, p.z.P);   // (the first pass loads P points a thread: the wider one)
     for (RzCols &g : p.zc) {
         g.n1h = s.n1h;
         g.n2 = s.n2;
