@@ -14,7 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(LIBDIR, "libpscfgpu.so")
-SOURCES = ["engine.cu", "sweep_rx_f64.cu", "sweep_rx_f32.cu", "noalloc.cu"]
+SOURCES = ["engine.cu", "sweep_rx3_f64.cu", "sweep_rx3_f32.cu", "sweep_rx2_f64.cu", "sweep_rx2_f32.cu", "noalloc.cu"]
 # compiled on their own, with extra flags: the graph-driven Anderson control
 # kernels round as the host iteration does only without multiply-add
 # contraction

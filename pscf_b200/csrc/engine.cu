@@ -535,14 +535,15 @@ static void create_engine(Engine &E, const pscfg_system *sys, int n_inst, int pr
     make_geom<double>(E, E.g64);
     if (precision != PSCFG_FP64) make_geom<float>(E, E.g32);
     {
-        std::vector<RxCol> cols(E.n[0] / 2 + 1);
-        if (rx_shape(E.dim, E.n, E.rx, cols.data())) {
+        const int nc = E.n[0] / 2 + 1;
+        std::vector<RxCol> cols(2 * nc);
+        if (rx_shape(E.dim, E.n, E.rx, cols.data(), false) && rx_shape(E.dim, E.n, E.rx, cols.data() + nc, true)) {
             RxCol *d = (RxCol *)E.dalloc(cols.size() * sizeof(RxCol));
             CK(cudaMemcpy(d, cols.data(), cols.size() * sizeof(RxCol), cudaMemcpyHostToDevice));
             for (int k = 0; k < 2; k++) {
                 const PlaneGeom &g = k ? E.g32 : E.g64;
-                E.rx.tb[k] = RxTables{g.rtw, g.col.tw, d};
-                E.rx.zc[k].cols = d;
+                E.rx.tb[k] = RxTables{g.rtw, g.col.tw, d + k * nc};
+                E.rx.zc[k].cols = d + k * nc;
                 E.rx.zc[k].twz = g.zp.tw;
             }
         }

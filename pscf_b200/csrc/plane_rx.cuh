@@ -123,10 +123,17 @@ struct RxCol {
 };
 
 // Rotation of the slots of a k1 group: with 8 values in a group only half
-// of them (kx <= n1/2) are columns, so odd groups start at the other half
-// and two groups fill the banks.
-__host__ __device__ __forceinline__ constexpr int rx_rot(int Q1, int k1) { return Q1 == 8 ? 4 * (k1 & 1) : 0; }
-__host__ __device__ __forceinline__ constexpr int rx_slot(int Q1, int k1, int k2) { return Q1 * k1 + (k2 + rx_rot(Q1, k1)) % Q1; }
+// of them (kx <= n1/2) are columns, so some groups start at the other half
+// and together fill the banks: 8 values of 16 bytes (every other group) or
+// 16 of 8 (every other two).
+template <typename T> __host__ __device__ __forceinline__ constexpr int rx_rot(int Q1, int k1)
+{
+    return Q1 == 8 ? 4 * ((sizeof(T) == 8 ? k1 : k1 >> 1) & 1) : 0;
+}
+template <typename T> __host__ __device__ __forceinline__ constexpr int rx_slot(int Q1, int k1, int k2)
+{
+    return Q1 * k1 + (k2 + rx_rot<T>(Q1, k1)) % Q1;
+}
 // line stride in complex values: n1 slots, two spare ones, odd
 __host__ __device__ __forceinline__ constexpr int rx_stride(int n1) { return (n1 + 2) | 1; }
 
@@ -237,7 +244,7 @@ template <typename T, typename SH> struct Rx {
             for (int w = threadIdx.x; w < nl * sh.P1; w += blockDim.x) {
                 const int k1 = dnl.div(w), l = w - nl * k1;
                 C *b = buf + line(l) * sh.LS + Q * k1;
-                const int rot = rx_rot(Q, k1);   // Q = 8: slot of k2 is k2 ^ rot
+                const int rot = rx_rot<T>(Q, k1);   // Q = 8: slot of k2 is k2 ^ rot
                 C v[Q];
                 if (S < 0) {
 #pragma unroll

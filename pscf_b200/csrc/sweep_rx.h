@@ -16,8 +16,9 @@ struct RxPlan {
     RzCols zc[2];
 };
 
-// Fills sh, z and the column table of a grid; false: a length without radices.
-bool rx_shape(int dim, const int n[3], RxPlan &p, RxCol *cols);
+// Fills sh, z and the column table (of one type) of a grid; false: a length
+// without radices.
+bool rx_shape(int dim, const int n[3], RxPlan &p, RxCol *cols, bool f32);
 
 // dim 2: steps [t0, t1) of every field
 template <typename T> int rx2_sweep(const RxPlan &p, cudaStream_t st, const SweepField<T> *f, int nf, int t0, int t1);

@@ -1,5 +1,5 @@
 // sweep_rx.inl -- launches of the plane_rx.cuh kernels for one type,
-// included by sweep_rx_f64.cu and sweep_rx_f32.cu.
+// included by the sweep_rx*.cu units (one per dimension and type).
 #include <algorithm>
 
 #include "../../include/pscf_gpu.h"
@@ -238,9 +238,10 @@ int rx3_stress(const RxPlan &p, cudaStream_t st, const StressJob<T> *jobs, int n
     });
 }
 
-#define RX_INSTANCES(T)                                                                                              \
+#define RX2_INSTANCES(T)                                                                                             \
     template int rx2_sweep<T>(const RxPlan &, cudaStream_t, const SweepField<T> *, int, int, int);                   \
-    template int rx2_stress<T>(const RxPlan &, cudaStream_t, const StressJob<T> *, int, int);                        \
+    template int rx2_stress<T>(const RxPlan &, cudaStream_t, const StressJob<T> *, int, int);
+#define RX3_INSTANCES(T)                                                                                             \
     template int rx3_planes<T>(const RxPlan &, int);                                                                 \
     template bool rx3_fits<T>(const RxPlan &);                                                                       \
     template int rx3_first<T>(const RxPlan &, cudaStream_t, const SweepField<T> *, int, int);                        \

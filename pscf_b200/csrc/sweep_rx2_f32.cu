@@ -1,8 +1,8 @@
-// plane_rx.cuh kernels in FP32.
+// plane_rx.cuh kernels for dim 2 in FP32.
 #include "sweep_rx.inl"
 
 namespace pscfg {
 
-RX_INSTANCES(float)
+RX2_INSTANCES(float)
 
 }  // namespace pscfg

@@ -1,4 +1,4 @@
-// plane_rx.cuh kernels in FP64, and the shapes they take.
+// plane_rx.cuh kernels for dim 2 in FP64, and the shapes all of them take.
 #include "sweep_rx.inl"
 
 namespace pscfg {
@@ -25,7 +25,7 @@ static bool split(int n, bool first_small, bool even, int &P, int &Q)
     return best < (1 << 30);
 }
 
-bool rx_shape(int dim, const int n[3], RxPlan &p, RxCol *cols)
+bool rx_shape(int dim, const int n[3], RxPlan &p, RxCol *cols, bool f32)
 {
     RxShape &s = p.sh;
     s.n1 = n[0];
@@ -43,7 +43,9 @@ bool rx_shape(int dim, const int n[3], RxPlan &p, RxCol *cols)
     s.dP2 = RDiv::of(s.P2);
     s.dn2 = RDiv::of(s.n2);
     int c = 0;
-    auto slot = [&](int kx) { return rx_slot(s.Q1, kx % s.P1, kx / s.P1); };
+    auto slot = [&](int kx) {
+        return f32 ? rx_slot<float>(s.Q1, kx % s.P1, kx / s.P1) : rx_slot<double>(s.Q1, kx % s.P1, kx / s.P1);
+    };
     auto add = [&](int kx) {
         RxCol &k = cols[c++];
         k.kx = (short)kx;
@@ -64,6 +66,6 @@ bool rx_shape(int dim, const int n[3], RxPlan &p, RxCol *cols)
     return true;
 }
 
-RX_INSTANCES(double)
+RX2_INSTANCES(double)
 
 }  // namespace pscfg
