@@ -2124,6 +2124,20 @@ static void stress_all(Engine &E, const std::vector<int> &act)
     }
 }
 
+// The stress of every instance, [n_inst][PSCFG_MAXCP], gathered on the device
+// for one copy.
+static void read_stress(Engine &E, double *out)
+{
+    const int ni = (int)E.inst.size();
+    std::vector<CopyJob> cj;
+    double *dst = E.dstage + (size_t)E.hpin_inst * 16;
+    for (int i = 0; i < ni; i++) cj.push_back(CopyJob{E.inst[i].stress_dev, dst + (size_t)i * 8, PSCFG_MAXCP});
+    copy_list(E, cj, 8);
+    CK(cudaMemcpyAsync(E.hst(0), dst, sizeof(double) * 8 * ni, cudaMemcpyDeviceToHost, E.st));
+    CK(cudaStreamSynchronize(E.st));
+    for (int i = 0; i < ni; i++) std::memcpy(out + (size_t)i * PSCFG_MAXCP, E.hst(i), sizeof(double) * PSCFG_MAXCP);
+}
+
 // ---------------------------------------------------------------------
 // Free energy (src/scf_mod.fp.f90:834-886)
 // ---------------------------------------------------------------------
@@ -3073,10 +3087,7 @@ static void am_results(Engine &E, AmRun &R, std::vector<pscfg_am_result> &res)
     std::vector<double> shost((size_t)ninst * PSCFG_MAXCP, 0.0);
     if (!R.prm.domain) {
         stress_all(E, all);
-        for (int i = 0; i < ninst; i++)
-            CK(cudaMemcpyAsync(&shost[(size_t)i * PSCFG_MAXCP], E.inst[i].stress_dev, sizeof(double) * PSCFG_MAXCP,
-                               cudaMemcpyDeviceToHost, E.st));
-        CK(cudaStreamSynchronize(E.st));
+        read_stress(E, shost.data());
     }
     res.resize(ninst);
     for (int i = 0; i < ninst; i++) {
@@ -3184,7 +3195,7 @@ static void adjoint_impl(Engine &E, const std::vector<int> &act, const std::vect
         std::vector<double> coef;   // [ns+1][MAXM] incl. phi/(L Q)
     };
     std::vector<Sweep> sw;
-    const int nct = red_ctas(nr);
+    int nct = red_ctas(nr);
     // coefficients, overlaps S_c
     std::vector<AdjOverlap> ov;
     std::vector<std::pair<int, int>> ov_ic;
@@ -3296,6 +3307,7 @@ static void adjoint_impl(Engine &E, const std::vector<int> &act, const std::vect
     } else {
         AdjOverlap *dov = E.upload(ov, off);
         off += ((ov.size() * sizeof(AdjOverlap) + 255) / 256) * 256;
+        nct = red_ctas(nr, (int)ov.size());   // (64 CTAs read a 64^3 contour's 843 MB in 2.24 ms)
         double *part = E.part((size_t)nct * ov.size());
         k_adj_overlap<T><<<dim3(nct, (unsigned)ov.size()), 256, 0, E.st>>>(dov, nr, part);
         E.launched();
@@ -4113,13 +4125,7 @@ int pscfg_stress(pscfg_engine *e, double *stress)
     std::vector<int> all(ni);
     for (int i = 0; i < ni; i++) all[i] = i;
     stress_all(E, all);
-    std::vector<CopyJob> cj;
-    double *dst = E.dstage + (size_t)E.hpin_inst * 16;
-    for (int i = 0; i < ni; i++) cj.push_back(CopyJob{E.inst[i].stress_dev, dst + (size_t)i * 8, PSCFG_MAXCP});
-    copy_list(E, cj, 8);
-    CK(cudaMemcpyAsync(E.hst(0), dst, sizeof(double) * 8 * ni, cudaMemcpyDeviceToHost, E.st));
-    CK(cudaStreamSynchronize(E.st));
-    for (int i = 0; i < ni; i++) std::memcpy(stress + (long)i * PSCFG_MAXCP, E.hst(i), sizeof(double) * PSCFG_MAXCP);
+    read_stress(E, stress);
     for (int i = 0; i < ni; i++)
         for (int b = E.inst[i].cell.ncp; b < PSCFG_MAXCP; b++) stress[(long)i * PSCFG_MAXCP + b] = 0.0;
     ABI_END(e)

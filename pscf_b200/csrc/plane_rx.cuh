@@ -143,8 +143,8 @@ __host__ __device__ __forceinline__ constexpr int rx_stride(int n1) { return (n1
 struct RxShape {
     static constexpr bool FIXED = false;
     static constexpr int PM = 10, QM = 16;
-    int n1, n2, n1h, P1, Q1, P2, Q2, HP, LS;
-    RDiv dQ1, dn1h, dQ2, dP2, dn2;
+    int n1, n2, n1h, nc, P1, Q1, P2, Q2, HP, LS;   // nc: columns without kx = n1/2
+    RDiv dQ1, dn1h, dnc, dQ2, dP2, dn2;
 };
 struct RxShape10 : RxShape {
     static constexpr int PM = 8, QM = 10;
@@ -152,10 +152,11 @@ struct RxShape10 : RxShape {
 // compile-time plane shape
 template <int N1, int N2, int P1_, int P2_> struct RxFixed {
     static constexpr bool FIXED = true;
-    static constexpr int n1 = N1, n2 = N2, n1h = N1 / 2 + 1, P1 = P1_, Q1 = N1 / P1_, P2 = P2_, Q2 = N2 / P2_,
+    static constexpr int n1 = N1, n2 = N2, n1h = N1 / 2 + 1, nc = (N1 + 1) / 2, P1 = P1_, Q1 = N1 / P1_, P2 = P2_, Q2 = N2 / P2_,
                          HP = (P2_ + 1) / 2, LS = rx_stride(N1);
     SDiv<N1 / P1_> dQ1;
     SDiv<N1 / 2 + 1> dn1h;
+    SDiv<(N1 + 1) / 2> dnc;
     SDiv<N2 / P2_> dQ2;
     SDiv<P2_> dP2;
     SDiv<N2> dn2;
@@ -264,6 +265,20 @@ template <typename T, typename SH> struct Rx {
         RX_Q(SH, Q1, go);
     }
 
+    // Item w of a column pass over nt groups -> (group t, column c): the nc
+    // columns of every group first (for powers of two whole warps on one
+    // group, aligned to the banks), then the column kx = n1/2 of each.
+    __device__ __forceinline__ static void col_item(const SH &sh, int w, int nt, int &t, int &c)
+    {
+        if (w < nt * sh.nc) {
+            t = sh.dnc.div(w);
+            c = w - sh.nc * t;
+        } else {
+            t = w - nt * sh.nc;
+            c = sh.nc;
+        }
+    }
+
     __device__ __forceinline__ static C sumc(C z, C zp) { return mk<T>(z.x + zp.x, z.y - zp.y); }    // z + conj zp
     __device__ __forceinline__ static C difc(C z, C zp) { return mk<T>(z.y + zp.y, zp.x - z.x); }    // -i (z - conj zp)
 
@@ -276,7 +291,8 @@ template <typename T, typename SH> struct Rx {
         auto go = [&](auto pc) {
             constexpr int P = decltype(pc)::value;
             for (int w = threadIdx.x; w < np * sh.Q2 * sh.n1h; w += blockDim.x) {
-                const int t = sh.dn1h.div(w), c = w - sh.n1h * t;
+                int t, c;
+                col_item(sh, w, np * sh.Q2, t, c);
                 const int pl = sh.dQ2.div(t), r = t - sh.Q2 * pl;
                 const RxCol col = ct[c];
                 C *b = buf + (pl * ld + r) * sh.LS;
@@ -322,7 +338,8 @@ template <typename T, typename SH> struct Rx {
         auto go = [&](auto pc) {
             constexpr int P = decltype(pc)::value;
             for (int w = threadIdx.x; w < np * sh.Q2 * sh.n1h; w += blockDim.x) {
-                const int t = sh.dn1h.div(w), c = w - sh.n1h * t;
+                int t, c;
+                col_item(sh, w, np * sh.Q2, t, c);
                 const int pl = sh.dQ2.div(t), r = t - sh.Q2 * pl;
                 const RxCol col = ct[c];
                 const bool real = col.pos == col.ppos;   // kx = 0 or n1/2: the rows' spectra are real there
@@ -381,7 +398,8 @@ template <typename T, typename SH> struct Rx {
             constexpr int Q = decltype(qc)::value;
             const int ng = (FP ? 2 : 1) * np * sh.P2;
             for (int w = threadIdx.x; w < ng * sh.n1h; w += blockDim.x) {
-                const int t = sh.dn1h.div(w), c = w - sh.n1h * t;
+                int t, c;
+                col_item(sh, w, ng, t, c);
                 const int u = sh.dP2.div(t), k1 = t - sh.P2 * u;
                 const int ab = FP ? (u & 1) : 0, pl = FP ? (u >> 1) : u;
                 const RxCol col = ct[c];
@@ -683,7 +701,8 @@ __global__ void __launch_bounds__(NT) k2x_stress(const StressJob<T> *jobs, SH sh
     auto dots = [&](auto qc) {
         constexpr int Q = decltype(qc)::value;
         for (int w = threadIdx.x; w < sh.P2 * sh.n1h; w += blockDim.x) {
-            const int k1 = sh.dn1h.div(w), c = w - sh.n1h * k1;
+            int k1, c;
+            X::col_item(sh, w, sh.P2, k1, c);
             const RxCol col = m.ct[c];
             const C *b0 = m.buf + Q * (k1 / 2) * sh.LS + ((k1 & 1) ? col.wpos : col.pos), *b1 = b0 + npair * sh.LS;
             C a[Q], b[Q];

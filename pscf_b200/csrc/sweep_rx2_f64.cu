@@ -32,6 +32,7 @@ bool rx_shape(int dim, const int n[3], RxPlan &p, RxCol *cols, bool f32)
     s.n2 = n[1];
     p.n3 = n[2];
     s.n1h = s.n1 / 2 + 1;
+    s.nc = (s.n1 + 1) / 2;
     p.plane = dim >= 2 && split(s.n1, true, false, s.P1, s.Q1) && split(s.n2, true, true, s.P2, s.Q2) &&
               s.n1 * s.n2 < 65536 / 2;
     if (!p.plane) return false;
@@ -39,6 +40,7 @@ bool rx_shape(int dim, const int n[3], RxPlan &p, RxCol *cols, bool f32)
     s.LS = rx_stride(s.n1);
     s.dQ1 = RDiv::of(s.Q1);
     s.dn1h = RDiv::of(s.n1h);
+    s.dnc = RDiv::of(s.nc);
     s.dQ2 = RDiv::of(s.Q2);
     s.dP2 = RDiv::of(s.P2);
     s.dn2 = RDiv::of(s.n2);
