@@ -449,6 +449,9 @@ template <typename T, typename SH> struct RxMem {
     __device__ __forceinline__ void *end(const SH &sh) const { return ct + sh.n1h; }
 };
 
+// Row stride of a real plane in shared memory: 8 (mod 16) values, so that the
+// two rows of a half warp lie on different banks.
+__host__ __device__ __forceinline__ constexpr int rx2_stride(int n1) { return n1 + (24 - n1 % 16) % 16; }
 // ---------------------------------------------------------------------
 // dim 2: a field's whole sweep in one CTA.  Per step one FP transform pair
 // (a = exp(-w ds/4) q with the filter ek2, b = exp(-w ds/2) q with ek1) and
@@ -462,9 +465,6 @@ template <typename T, typename SH> struct RxMem {
 // ---------------------------------------------------------------------
 // TAB: the current block's tables (exp(-w ds/4), and both filters in column
 // order) sit in shared memory too: for launches of at most one CTA per SM.
-// Row stride of its real planes: 8 (mod 16) values, so that the two rows of
-// a half warp lie on different banks.
-__host__ __device__ __forceinline__ constexpr int rx2_stride(int n1) { return n1 + (24 - n1 % 16) % 16; }
 template <typename T> __host__ __device__ constexpr size_t rx2_smem(int n1, int n2, bool tab)
 {
     return (rx_smem<T>(n1, n2, n2) + 15) / 16 * 16 +
@@ -650,6 +650,221 @@ __global__ void __launch_bounds__(NT, MB)
     }
 }
 
+
+// ---------------------------------------------------------------------
+// dim 2: a field's whole sweep by a cluster of two CTAs: rank 0 makes the
+// full steps q1, rank 1 the two half steps and the combination.  Each works
+// on RP lines with the filter applied between the two column passes in
+// registers (6 barriers a transform pair).  q1 crosses through the slice that
+// the step is about to write, q through that slice once it is written; two
+// cluster barriers a step order them, and rank 0 has half of rank 1's work,
+// so that neither wait is long.
+// Bound: rank 1's chain of 12 barriers and exchanges a step, or shared memory
+// wavefronts where several CTAs share an SM.
+// TAB: the current block's tables (exp(-w ds/4) and the rank's filter in
+// column order) sit in shared memory too: for launches of at most one CTA
+// per SM.
+// grid = 2 nfields.
+// ---------------------------------------------------------------------
+template <typename T> __host__ __device__ constexpr size_t rx2_pair_smem(int n1, int n2, int npair, bool tab)
+{
+    return (rx_smem<T>(n1, n2, npair) + 15) / 16 * 16 +
+           (tab ? sizeof(T) * ((size_t)rx2_stride(n1) * n2 + (n1 / 2 + 1) * n2) : 0);
+}
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+template <typename T, typename SH, int NT, int MB, bool TAB>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NT, MB)
+    k2x_pair(const SweepField<T> *fields, SH sh, RxTables tb, int t0, int t1)
+{
+    using X = Rx<T, SH>;
+    using C = cx<T>;
+    const SweepField<T> &f = fields[blockIdx.x >> 1];
+    const int rank = blockIdx.x & 1, npair = sh.Q2 * sh.HP;
+    const RxMem<T, SH> m(sh, tb, npair);
+    const int nr = sh.n1 * sh.n2, nkc = sh.n1h * sh.n2, QS = rx2_stride(sh.n1);
+    T *te2 = (T *)(((size_t)m.end(sh) + 15) / 16 * 16), *tek = te2 + QS * sh.n2;   // (TAB)
+    const T rn = (T)(2.0 * nr), rr = (T)(1.0 / (2.0 * nr)), rt = (T)(1.0 / 3.0);
+    const RDiv dpair = RDiv::of(npair), dn1 = RDiv::of(sh.n1);
+    auto same = [](int l) { return l; };
+    int blk, src, dst;
+    if (!step_slices(f, t0, blk, src, dst)) return;   // the same for the whole cluster
+    __syncthreads();
+    // f(P, line, r, y0's offset + r in a global plane, in a padded one, y1 exists)
+    auto items = [&](auto f2) {
+        auto go = [&](auto pc) {
+            for (int w = threadIdx.x; w < npair * sh.Q1; w += blockDim.x) {
+                const int l = sh.dQ1.div(w), r = w - sh.Q1 * l, y0 = l + sh.Q2 * sh.dQ2.div(l);   // r2 + 2 j Q2
+                f2(pc, m.buf + l * sh.LS, r, y0 * sh.n1 + r, y0 * QS + r, y0 + sh.Q2 < sh.n2);
+            }
+        };
+        RX_P(SH, P1, go);
+    };
+    // P values of rows y0 and y1 of a global plane (or of the padded table)
+    auto load2 = [&](auto pc, const T *p, int row, bool two, T *a, T *b, bool cg) {
+        constexpr int P = decltype(pc)::value;
+#pragma unroll
+        for (int i = 0; i < P; i++) {
+            a[i] = cg ? __ldcg(p + sh.Q1 * i) : p[sh.Q1 * i];
+            b[i] = !two ? (T)0 : cg ? __ldcg(p + sh.Q2 * row + sh.Q1 * i) : p[sh.Q2 * row + sh.Q1 * i];
+        }
+    };
+    auto load_e = [&](auto pc, const T *e2, bool table, int g, int pd, bool two, T *a, T *b) {
+        if (table) load2(pc, te2 + pd, QS, two, a, b, false);
+        else load2(pc, e2 + g, sh.n1, two, a, b, false);
+    };
+    // transform, filter, transform back, up to the real-space row passes
+    auto conv = [&](const T *ekt) {
+        __syncthreads();
+        X::template rows2<-1>(sh, m.buf, npair, dpair, same);
+        __syncthreads();
+        X::template cols_fwd1<false, 1>(sh, m.buf, 1, npair, m.ct, m.tw2);
+        __syncthreads();
+        X::template cols2<false, 1>(sh, m.buf, 1, npair, m.ct, [&](auto qc, int c, int kx, int, int, int k1, C *s, C *v) {
+            constexpr int Q = decltype(qc)::value;
+            const T *ek = ekt + (TAB ? c : kx) + sh.n1h * k1;
+            T e[Q];
+#pragma unroll
+            for (int k = 0; k < Q; k++) e[k] = TAB ? ek[sh.n1h * sh.P2 * k] : __ldg(ek + sh.n1h * sh.P2 * k);
+#pragma unroll
+            for (int n = 0; n < Q; n++) v[n] = s[n * sh.LS];
+            Dft<Q, -1, T>::run(v);
+#pragma unroll
+            for (int k = 0; k < Q; k++) v[k] = scale(v[k], e[k]);
+            Dft<Q, 1, T>::run(v);
+#pragma unroll
+            for (int n = 0; n < Q; n++) s[n * sh.LS] = v[n];
+        });
+        __syncthreads();
+        X::template cols_inv1<false, 1>(sh, m.buf, 1, npair, m.ct, m.tw2);
+        __syncthreads();
+        X::template rows2<1>(sh, m.buf, npair, dpair, same);
+        __syncthreads();
+    };
+    int cur = -1;
+    for (int t = t0; t < t1; t++) {
+        if (!step_slices(f, t, blk, src, dst)) break;
+        const T *e2 = f.eo2[blk], *ekt = rank ? f.ek2[blk] : f.ek1[blk];
+        if (TAB) {
+            if (blk != cur) {
+                cur = blk;
+                __syncthreads();
+                for (int i = threadIdx.x; i < nr; i += blockDim.x) te2[i + (QS - sh.n1) * dn1.div(i)] = e2[i];
+                for (int i = threadIdx.x; i < nkc; i += blockDim.x) {
+                    const int ky = sh.dn1h.div(i);
+                    tek[i] = ekt[m.ct[i - sh.n1h * ky].kx + sh.n1h * ky];
+                }
+                __syncthreads();
+            }
+            ekt = tek;
+        }
+        T *out = dst_slice(f, dst, nr);
+        if (rank == 0) {
+            const T *q = src_slice(f, src, nr);
+            items([&](auto pc, C *b, int r, int g, int pd, bool two) {
+                constexpr int P = decltype(pc)::value;
+                T q0[P], q1[P], ea[P], eb[P];
+                load2(pc, q + g, sh.n1, two, q0, q1, true);
+                load_e(pc, e2, TAB, g, pd, two, ea, eb);
+                C v[P];
+#pragma unroll
+                for (int i = 0; i < P; i++) v[i] = mk<T>(ea[i] * (ea[i] * q0[i]), eb[i] * (eb[i] * q1[i]));
+                X::template row_fwd1<P>(sh, b, r, v, m.tw1);
+            });
+            conv(ekt);
+            items([&](auto pc, C *b, int r, int g, int pd, bool two) {
+                constexpr int P = decltype(pc)::value;
+                T ea[P], eb[P];
+                load_e(pc, e2, TAB, g, pd, two, ea, eb);
+                C v[P];
+                X::template row_inv1<P>(sh, b, r, v, m.tw1);
+                auto put = [&](T *p) {
+#pragma unroll
+                    for (int i = 0; i < P; i++) {
+                        p[g + sh.Q1 * i] = div_by(ea[i] * ea[i] * v[i].x, rn, rr);
+                        if (two) p[g + sh.Q2 * sh.n1 + sh.Q1 * i] = div_by(eb[i] * eb[i] * v[i].y, rn, rr);
+                    }
+                };
+                put(out);
+                if (f.q1) put(f.q1);
+            });
+            cluster_arrive();   // q1 is in the destination slice
+            cluster_wait();
+            cluster_arrive();
+            cluster_wait();     // ... and now q
+        } else {
+            if (t == t0) {
+                const T *q = src_slice(f, src, nr);
+                items([&](auto pc, C *b, int r, int g, int pd, bool two) {
+                    constexpr int P = decltype(pc)::value;
+                    T q0[P], q1[P], ea[P], eb[P];
+                    load2(pc, q + g, sh.n1, two, q0, q1, false);
+                    load_e(pc, e2, TAB, g, pd, two, ea, eb);
+                    C v[P];
+#pragma unroll
+                    for (int i = 0; i < P; i++) v[i] = mk<T>(ea[i] * q0[i], eb[i] * q1[i]);
+                    X::template row_fwd1<P>(sh, b, r, v, m.tw1);
+                });
+            }
+            cluster_arrive();
+            conv(ekt);
+            items([&](auto pc, C *b, int r, int g, int pd, bool two) {
+                constexpr int P = decltype(pc)::value;
+                T ea[P], eb[P];
+                load_e(pc, e2, TAB, g, pd, two, ea, eb);
+                C v[P];
+                X::template row_inv1<P>(sh, b, r, v, m.tw1);
+#pragma unroll
+                for (int i = 0; i < P; i++) {
+                    v[i] = mk<T>(div_by(ea[i] * ea[i] * v[i].x, rn, rr), two ? div_by(eb[i] * eb[i] * v[i].y, rn, rr) : (T)0);
+                    if (f.h_out) {
+                        f.h_out[g + sh.Q1 * i] = v[i].x;
+                        if (two) f.h_out[g + sh.Q2 * sh.n1 + sh.Q1 * i] = v[i].y;
+                    }
+                }
+                X::template row_fwd1<P>(sh, b, r, v, m.tw1);
+            });
+            conv(ekt);
+            int blk2, src2, dst2;
+            const bool next = t + 1 < t1 && step_slices(f, t + 1, blk2, src2, dst2);
+            const bool table = TAB && next && blk2 == blk;
+            const T *n2 = next ? f.eo2[blk2] : nullptr;
+            cluster_wait();     // q1 is in the destination slice
+            items([&](auto pc, C *b, int r, int g, int pd, bool two) {
+                constexpr int P = decltype(pc)::value;
+                // (all loads ahead of the stores, which the compiler must
+                // assume to alias them)
+                T q0[P], q1[P], ea[P], eb[P];
+                load2(pc, out + g, sh.n1, two, q0, q1, true);
+                load_e(pc, e2, TAB, g, pd, two, ea, eb);
+                C v[P];
+                X::template row_inv1<P>(sh, b, r, v, m.tw1);
+#pragma unroll
+                for (int i = 0; i < P; i++) {
+                    const T qa = div_by(ea[i] * v[i].x, rn, rr), qb = div_by(eb[i] * v[i].y, rn, rr);
+                    if (f.q2_out) {
+                        f.q2_out[g + sh.Q1 * i] = qa;
+                        if (two) f.q2_out[g + sh.Q2 * sh.n1 + sh.Q1 * i] = qb;
+                    }
+                    q0[i] = div_by((T)4 * qa - q0[i], (T)3, rt);
+                    q1[i] = div_by((T)4 * qb - q1[i], (T)3, rt);
+                }
+                if (next && n2 != e2) load_e(pc, n2, table, g, pd, two, ea, eb);
+#pragma unroll
+                for (int i = 0; i < P; i++) {
+                    out[g + sh.Q1 * i] = q0[i];
+                    if (two) out[g + sh.Q2 * sh.n1 + sh.Q1 * i] = q1[i];
+                    v[i] = mk<T>(ea[i] * q0[i], two ? eb[i] * q1[i] : (T)0);
+                }
+                if (next) X::template row_fwd1<P>(sh, b, r, v, m.tw1);
+            });
+            cluster_arrive();
+            cluster_wait();
+        }
+    }
+}
 
 // First forward row passes of the RP lines of one real plane: pairs of rows
 // of src into the lines from `line0` on.

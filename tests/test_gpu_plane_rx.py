@@ -50,6 +50,24 @@ def test_boxes_match_oracle(n, precision, tol):
     check(diblock(3, n, "orthorhombic", [1.6, 2.1, 1.9], fA=0.35, ds=0.1, b=(1.0, 1.3)), precision, tol)
 
 
+@pytest.mark.parametrize("count", [37, 38, 75])
+def test_planes_of_batches_match_single_ones(count):
+    """The 2-D sweep's three forms (by the number of fields) agree to
+    roundoff: 2 x 37 fields with two CTAs each, 2 x 38 with one, 2 x 75 with
+    two CTAs to an SM."""
+    for n in ([64, 64], [18, 15]):
+        s = diblock(2, n, "rectangular", [1.6, 2.1], fA=0.35, ds=0.1)
+        w = omega_guess(s, 4, 2.0)
+        e1 = Engine([s], FP64)
+        rho1, q1 = e1.density(w[None])
+        e = Engine([s] * count, FP64)
+        rho, q = e.density(np.stack([w] * count))
+        for i in (0, count - 1):
+            assert rel_err(rho[i], rho1[0]) < 1e-12 and rel_err(q[i, :1], q1[0, :1]) < 1e-12
+        e.close()
+        e1.close()
+
+
 def test_stress_of_slices_of_very_different_size():
     """qf and qr of one slice differ by e^30 at the chain's ends: neither may
     carry the other's rounding (relative 1e-10, as for the older kernels)."""
