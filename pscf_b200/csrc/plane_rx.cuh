@@ -162,6 +162,22 @@ template <int N1, int N2, int P1_, int P2_> struct RxFixed {
     SDiv<N2> dn2;
 };
 
+// Column c of a fixed shape (even Q1: every k1 group holds Q1 / 2 columns, kx
+// = n1/2 follows them), as in the run-time shapes' tables.
+template <typename T, typename SH> __device__ __forceinline__ RxCol rx_fixed_col(int c)
+{
+    constexpr int P = SH::P1, Q = SH::Q1, H = Q / 2;
+    static_assert(Q % 2 == 0, "columns in whole groups");
+    const int k1 = c == SH::nc ? 0 : c / H, k2 = c == SH::nc ? H : c % H;
+    const int q1 = k1 ? P - k1 : 0, q2 = k1 ? Q - 1 - k2 : (Q - k2) % Q;
+    RxCol r;
+    r.kx = (short)(k1 + P * k2);
+    r.pos = (short)rx_slot<T>(Q, k1, k2);
+    r.ppos = (short)rx_slot<T>(Q, q1, q2);
+    r.wpos = c == 0 ? (short)SH::n1 : c == SH::nc ? (short)(SH::n1 + 1) : r.ppos;
+    return r;
+}
+
 template <int V> struct RxInt {
     static constexpr int value = V;
 };
@@ -279,6 +295,12 @@ template <typename T, typename SH> struct Rx {
         }
     }
 
+    __device__ __forceinline__ static RxCol column(const RxCol *ct, int c)
+    {
+        if constexpr (SH::FIXED) return rx_fixed_col<T, SH>(c);
+        else return ct[c];
+    }
+
     __device__ __forceinline__ static C sumc(C z, C zp) { return mk<T>(z.x + zp.x, z.y - zp.y); }    // z + conj zp
     __device__ __forceinline__ static C difc(C z, C zp) { return mk<T>(z.y + zp.y, zp.x - z.x); }    // -i (z - conj zp)
 
@@ -294,7 +316,7 @@ template <typename T, typename SH> struct Rx {
                 int t, c;
                 col_item(sh, w, np * sh.Q2, t, c);
                 const int pl = sh.dQ2.div(t), r = t - sh.Q2 * pl;
-                const RxCol col = ct[c];
+                const RxCol col = column(ct, c);
                 C *b = buf + (pl * ld + r) * sh.LS;
                 if constexpr (FP) {
                     C a[P], d[P];
@@ -341,7 +363,7 @@ template <typename T, typename SH> struct Rx {
                 int t, c;
                 col_item(sh, w, np * sh.Q2, t, c);
                 const int pl = sh.dQ2.div(t), r = t - sh.Q2 * pl;
-                const RxCol col = ct[c];
+                const RxCol col = column(ct, c);
                 const bool real = col.pos == col.ppos;   // kx = 0 or n1/2: the rows' spectra are real there
                 C *b = buf + (pl * ld + r) * sh.LS;
                 auto put = [&](C *s, C a, C d) {
@@ -402,7 +424,7 @@ template <typename T, typename SH> struct Rx {
                 col_item(sh, w, ng, t, c);
                 const int u = sh.dP2.div(t), k1 = t - sh.P2 * u;
                 const int ab = FP ? (u & 1) : 0, pl = FP ? (u >> 1) : u;
-                const RxCol col = ct[c];
+                const RxCol col = column(ct, c);
                 // FP: lines Q2 k1 + n; RP: lines (k1 / 2) Q2 LSTEP + n
                 C *s = buf + (pl * ld + (FP ? Q * k1 : Q * LSTEP * (k1 / 2))) * sh.LS +
                        ((FP ? ab : (k1 & 1)) ? col.wpos : col.pos);
@@ -918,7 +940,7 @@ __global__ void __launch_bounds__(NT) k2x_stress(const StressJob<T> *jobs, SH sh
         for (int w = threadIdx.x; w < sh.P2 * sh.n1h; w += blockDim.x) {
             int k1, c;
             X::col_item(sh, w, sh.P2, k1, c);
-            const RxCol col = m.ct[c];
+            const RxCol col = X::column(m.ct, c);
             const C *b0 = m.buf + Q * (k1 / 2) * sh.LS + ((k1 & 1) ? col.wpos : col.pos), *b1 = b0 + npair * sh.LS;
             C a[Q], b[Q];
 #pragma unroll
@@ -1023,17 +1045,15 @@ __global__ void __launch_bounds__(NT, MB)
     using X = Rx<T, SH>;
     using C = cx<T>;
     const SweepField<T> &f = fields[blockIdx.y];
-    int blk, src, dst;
-    if (!step_slices(f, t, blk, src, dst)) return;
     const int z0 = blockIdx.x * ppc, np = min(ppc, n3 - z0), npl = sh.n1 * sh.n2, npair = sh.Q2 * sh.HP;
-    const RxMem<T, SH> m(sh, tb, ppc * npair);
-    const T *e2 = f.eo2[blk] + (long)z0 * npl;
-    T *ho = f.h_out ? f.h_out + (long)z0 * npl : nullptr;
     C *S = f.S2 + (long)z0 * sh.n2 * sh.n1h;
+    const RxMem<T, SH> m(sh, tb, ppc * npair);
     const T rn = (T)(2.0 * npl * n3), rr = (T)(1.0 / (2.0 * npl * n3));
     const RDiv dl = RDiv::of(np * npair), dpair = RDiv::of(npair);
     auto same = [](int l) { return l; };
-    __syncthreads();
+    // (the spectrum's loads go out before the step's descriptor is read; a
+    // field past its last step stops after them)
+    if (!SH::FIXED) __syncthreads();
     X::template cols2<false, 1>(sh, m.buf, np, npair, m.ct, [&](auto qc, int c, int, int, int pl, int k1, C *s, C *v) {
         constexpr int Q = decltype(qc)::value;
         const C *d = S + (long)(pl * sh.n2 + k1) * sh.n1h + c;
@@ -1043,6 +1063,10 @@ __global__ void __launch_bounds__(NT, MB)
 #pragma unroll
         for (int n = 0; n < Q; n++) s[n * sh.LS] = v[n];
     });
+    int blk, src, dst;
+    if (!step_slices(f, t, blk, src, dst)) return;
+    const T *e2 = f.eo2[blk] + (long)z0 * npl;
+    T *ho = f.h_out ? f.h_out + (long)z0 * npl : nullptr;
     __syncthreads();
     X::template cols_inv1<false, 1>(sh, m.buf, np, npair, m.ct, m.tw2);
     __syncthreads();
@@ -1099,20 +1123,12 @@ __global__ void __launch_bounds__(NT, MB)
     using X = Rx<T, SH>;
     using C = cx<T>;
     const SweepField<T> &f = fields[blockIdx.y];
-    int blk, src, dst;
-    if (!step_slices(f, t, blk, src, dst)) return;
     const int z0 = blockIdx.x * ppc, np = min(ppc, n3 - z0), npl = sh.n1 * sh.n2;
-    const RxMem<T, SH> m(sh, tb, ppc * sh.n2);
     const long po = (long)z0 * npl, so = (long)z0 * sh.n2 * sh.n1h;
-    const T *e2 = f.eo2[blk] + po;
-    T *out = dst_slice(f, dst, (long)npl * n3) + po;
-    T *q1o = f.h_out ? f.q1 + po : nullptr, *q2o = f.h_out && f.q2_out ? f.q2_out + po : nullptr;
-    int blk2, src2, dst2;
-    const bool next = step_slices(f, t + 1, blk2, src2, dst2);   // the same for the whole CTA
-    const T *n2 = f.eo2[next ? blk2 : blk] + po;
     const C *sa = f.S2 + so, *sb = f.S1 + so;
+    const RxMem<T, SH> m(sh, tb, ppc * sh.n2);
     const T rn = (T)(6.0 * npl * n3), rr = (T)(1.0 / (6.0 * npl * n3));
-    __syncthreads();
+    if (!SH::FIXED) __syncthreads();
     X::template cols2<true, 1>(sh, m.buf, np, sh.n2, m.ct, [&](auto qc, int c, int, int ab, int pl, int k1, C *s, C *v) {
         constexpr int Q = decltype(qc)::value;
         const C *d = (ab ? sb : sa) + (long)(pl * sh.n2 + k1) * sh.n1h + c;
@@ -1122,6 +1138,13 @@ __global__ void __launch_bounds__(NT, MB)
 #pragma unroll
         for (int n = 0; n < Q; n++) s[n * sh.LS] = v[n];
     });
+    int blk, src, dst, blk2, src2, dst2;
+    if (!step_slices(f, t, blk, src, dst)) return;   // (as in k3v_mid)
+    const T *e2 = f.eo2[blk] + po;
+    T *out = dst_slice(f, dst, (long)npl * n3) + po;
+    T *q1o = f.h_out ? f.q1 + po : nullptr, *q2o = f.h_out && f.q2_out ? f.q2_out + po : nullptr;
+    const bool next = step_slices(f, t + 1, blk2, src2, dst2);   // the same for the whole CTA
+    const T *n2 = f.eo2[next ? blk2 : blk] + po;
     __syncthreads();
     X::template cols_inv1<true, 1>(sh, m.buf, np, sh.n2, m.ct, m.tw2);
     __syncthreads();
@@ -1236,24 +1259,28 @@ __global__ void __launch_bounds__(NT, MB) k3v_zconv(const SweepField<T> *fields,
 {
     using C = cx<T>;
     const SweepField<T> &f = fields[blockIdx.y];
-    int blk, src, dst;
-    if (!step_slices(f, t, blk, src, dst)) return;
     const int sel = which == 3 ? (int)blockIdx.z + 1 : which;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *buf = (C *)smem_raw, *tw = buf + sh.n3 * TC;
     const int ncol = g.n1h * g.n2, c = threadIdx.x % TC, col = blockIdx.x * TC + c, r0 = threadIdx.x / TC;
-    constexpr int NR = NT / TC;
+    constexpr int NR = NT / TC;   // at least P and Q: one item a thread and pass
     const bool ok = col < ncol;
     C *S = ((sel == 1) ? f.S1 : f.S2) + (ok ? col : 0);
-    for (int i = threadIdx.x; i < sh.n3; i += NT) tw[i] = ((const C *)g.twz)[i];
-    const int ky = g.dn1h.div(ok ? col : 0), kx = g.cols[(ok ? col : 0) - ky * g.n1h].kx;
-    __syncthreads();
+    int blk, src, dst;
+    bool live = true;
     auto first = [&](auto pc) {
         constexpr int P = decltype(pc)::value;
-        for (int r = r0; r < sh.Q; r += NR) {
-            C v[P];
+        const int r = r0;
+        C v[P];
+        // (the loads go out before the tables and the step's descriptor are read)
+        if (r < sh.Q) {
 #pragma unroll
             for (int i = 0; i < P; i++) v[i] = ok ? S[(long)(sh.Q * i + r) * ncol] : mk<T>((T)0, (T)0);
+        }
+        for (int i = threadIdx.x; i < sh.n3; i += NT) tw[i] = ((const C *)g.twz)[i];
+        live = step_slices(f, t, blk, src, dst);
+        __syncthreads();
+        if (r < sh.Q && live) {
             Dft<P, -1, T>::run(v);
             C *b = buf + r * TC + c;
             b[0] = v[0];
@@ -1262,6 +1289,8 @@ __global__ void __launch_bounds__(NT, MB) k3v_zconv(const SweepField<T> *fields,
         }
     };
     RX_Q(ZS, P, first);
+    if (!live) return;   // a field past its last step, the same for the whole CTA
+    const int ky = g.dn1h.div(ok ? col : 0), kx = g.cols[(ok ? col : 0) - ky * g.n1h].kx;
     __syncthreads();
     const T *ekf = f.ekf[blk];
     const T *ek = ((sel == 1) ? f.ek1[blk] : f.ek2[blk]) + kx + (long)g.n1h * ky;

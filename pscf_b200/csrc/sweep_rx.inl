@@ -124,7 +124,7 @@ template <typename T, typename F> static int with_plane(const RxPlan &p, int cta
 }
 // f(shape, RxInt<columns of a tile>, RxInt<threads>, RxInt<CTAs per SM of the
 // filter pass>), for nf spectra: half as wide where the wide tiles would
-// leave SMs idle
+// leave SMs idle.  Threads / columns is at least P and Q.
 template <typename T, typename F> static int with_line(const RxPlan &p, int nf, F f)
 {
     constexpr bool F32 = sizeof(T) == 4;
@@ -144,6 +144,14 @@ template <typename T, typename F> static int with_line(const RxPlan &p, int nf, 
     if (q <= 8) return f(RzShape10{p.z}, RxInt<32>(), RxInt<256>(), RxInt<3>());
     if (q <= 10) return f(RzShape10{p.z}, RxInt<16>(), RxInt<160>(), RxInt<4>());
     return f(p.z, RxInt<16>(), RxInt<256>(), RxInt<2>());
+}
+
+// the same for the stress pass, whose two tiles have to leave room for several
+// CTAs per SM
+template <typename T, typename F> static int with_stress_line(const RxPlan &p, F f)
+{
+    if (p.z.n3 == 224 && sizeof(T) == 8) return f(RzFixed<224, 16>(), RxInt<8>(), RxInt<128>(), RxInt<3>());
+    return with_line<T>(p, 1 << 20, f);
 }
 
 template <typename T> static int fp_threads(const RxShape &s, int ppc, int most)
@@ -213,7 +221,7 @@ template <typename T> int rx3_step(const RxPlan &p, cudaStream_t st, const Sweep
 template <typename T> int rx3_stress_tiles(const RxPlan &p)
 {
     if (!rx3_fits<T>(p)) return 0;
-    return with_line<T>(p, 1 << 20, [&](auto, auto tc, auto, auto) {
+    return with_stress_line<T>(p, [&](auto, auto tc, auto, auto) {
         constexpr int TC = decltype(tc)::value;
         return rz_smem<T>(p.n3, TC, 2) <= SMEM_MOST - 1024 ? (p.sh.n1h * p.sh.n2 + TC - 1) / TC : 0;
     });
@@ -235,7 +243,7 @@ int rx3_stress(const RxPlan &p, cudaStream_t st, const StressJob<T> *jobs, int n
         return 1;
     });
     if (rc < 0) return -1;
-    return with_line<T>(p, 1 << 20, [&](auto z, auto tc, auto nt, auto) {
+    return with_stress_line<T>(p, [&](auto z, auto tc, auto nt, auto) {
         constexpr int TC = decltype(tc)::value, NT = decltype(nt)::value;
         auto *k = k3v_stress_z<T, decltype(z), TC, NT>;
         RX_LAUNCH(k, dim3((p.sh.n1h * p.sh.n2 + TC - 1) / TC, cnt, njobs), NT, rz_smem<T>(p.n3, TC, 2), st, jobs, z,
