@@ -1200,19 +1200,19 @@ static void run_sweeps(Engine &E, const std::vector<int> &act)
             }
         }
         if (ortho) {
+            // (qf and qr of a chain share them)
             for (int i : act) {
                 Inst &I = E.inst[i];
                 for (int c = 0; c < I.sys.n_chain; c++)
-                    for (int d = 0; d < 2; d++)
-                        for (int b = 0; b < I.sys.n_block[c]; b++) {
-                            const double kb = I.sys.kuhn[I.sys.block_monomer[c][b]];
-                            if (E.amg) {
-                                ekj.push_back(EkfJob{E.amg_G[i], I.bds[c][b] * kb * kb, nullptr});
-                                ekf.resize(ekf.size() + 2 * (size_t)L3, (T)0);
-                            } else {
-                                append_ek_factors<T>(E, I.cell, I.bds[c][b] * kb * kb, ekf);
-                            }
+                    for (int b = 0; b < I.sys.n_block[c]; b++) {
+                        const double kb = I.sys.kuhn[I.sys.block_monomer[c][b]];
+                        if (E.amg) {
+                            ekj.push_back(EkfJob{E.amg_G[i], I.bds[c][b] * kb * kb, nullptr});
+                            ekf.resize(ekf.size() + 2 * (size_t)L3, (T)0);
+                        } else {
+                            append_ek_factors<T>(E, I.cell, I.bds[c][b] * kb * kb, ekf);
                         }
+                    }
             }
         }
     }
@@ -1227,8 +1227,8 @@ static void run_sweeps(Engine &E, const std::vector<int> &act)
         }
         T *dtab = E.upload(ekf, off_tab);
         size_t k = 0;
-        for (auto &f : fl)
-            for (int b = 0; b < f.nblk; b++, k += 2 * (size_t)L3) f.ekf[b] = dtab + k;
+        for (size_t j = 0; j < fl.size(); j += 2)   // fl holds a chain's qf and qr one after the other
+            for (int b = 0; b < fl[j].nblk; b++, k += 2 * (size_t)L3) fl[j].ekf[b] = fl[j + 1].ekf[b] = dtab + k;
         if (!ekj.empty()) {
             for (size_t j = 0; j < ekj.size(); j++) ekj[j].out = dtab + j * 2 * (size_t)L3;
             EkfJob *dj = E.upload(ekj, off_ekj);
@@ -1333,7 +1333,7 @@ static void run_contour(Engine &E, const std::vector<int> &act)
         E.launched();
         double **dq = (double **)E.upload(qout, off);
         off += ((qout.size() * sizeof(void *) + 255) / 256) * 256;
-        k_final_sum_ptr<<<(unsigned)((qp.size() + 127) / 128), 128, 0, E.st>>>(part, nct, (double)E.nr, dq, (int)qp.size());
+        k_final_sum_ptr<<<(unsigned)((qp.size() + 3) / 4), 128, 0, E.st>>>(part, nct, (double)E.nr, dq, (int)qp.size());
         E.launched();
     }
     // solvents (src/scf_mod.fp.f90:193-200, 251-295): Q_s = <exp(-v w)>,
@@ -1376,7 +1376,7 @@ static void run_contour(Engine &E, const std::vector<int> &act)
         double *part = E.part((size_t)nct * sj.size());
         k_solvent_boltz_partial<<<dim3(nct, (unsigned)sj.size()), 256, 0, E.st>>>(dsj0, E.nr, part);
         E.launched();
-        k_final_sum_ptr<<<(unsigned)((sj.size() + 127) / 128), 128, 0, E.st>>>(part, nct, (double)E.nr, dqs, (int)sj.size());
+        k_final_sum_ptr<<<(unsigned)((sj.size() + 3) / 4), 128, 0, E.st>>>(part, nct, (double)E.nr, dqs, (int)sj.size());
         E.launched();
         k_solvent_rho<<<(unsigned)std::min<long>((E.nr + 255) / 256, 1024), 256, 0, E.st>>>(dsj0, (int)sj.size(), E.nr);
         E.launched();
@@ -2210,7 +2210,7 @@ static void fe_spectral(Engine &E, const std::vector<int> &which, double *hout, 
         k_fe_spectral<<<dim3(nct, cn), 256, 0, E.st>>>(dj, E.nk, E.n[0], part);
         E.launched();
         const double rn2 = (double)E.nr * (double)E.nr;
-        k_final_sum<<<(unsigned)((cn + 127) / 128), 128, 0, E.st>>>(part, nct, rn2, E.d_small, cn);
+        k_final_sum<<<(unsigned)((cn + 3) / 4), 128, 0, E.st>>>(part, nct, rn2, E.d_small, cn);
         E.launched();
         CK(cudaMemcpyAsync(hout + c0, E.d_small, sizeof(double) * cn,
                            dev_out ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, E.st));
@@ -2256,7 +2256,7 @@ static void free_energy_all(Engine &E, const std::vector<int> &act, std::vector<
         double *part = E.part((size_t)nct * fj.size());
         k_fe_partial<<<dim3(nct, (unsigned)fj.size()), 256, 0, E.st>>>(dj, E.nr, part);
         E.launched();
-        k_final_sum<<<(unsigned)((fj.size() + 127) / 128), 128, 0, E.st>>>(part, nct, (double)E.nr, E.d_small, (int)fj.size());
+        k_final_sum<<<(unsigned)((fj.size() + 3) / 4), 128, 0, E.st>>>(part, nct, (double)E.nr, E.d_small, (int)fj.size());
         E.launched();
         CK(cudaMemcpyAsync(hfe, E.d_small, sizeof(double) * fj.size(), kind, E.st));
     }
@@ -2398,7 +2398,7 @@ static void symmetrize_omega(Engine &E, const std::vector<int> &which)
     }
     if (jobs.empty()) return;
     SymJob *dj = E.upload(jobs, E.geom_off + ((size_t)1 << 20));
-    dim3 grid((unsigned)std::max(1, std::min((maxorb + 127) / 128, 256)), (unsigned)jobs.size());
+    dim3 grid((unsigned)std::max(1, std::min((maxorb * SYM_LANES + 127) / 128, 1024)), (unsigned)jobs.size());
     k_symmetrize<<<grid, 128, 0, E.st>>>(dj, E.nr);
     E.launched();
 }
@@ -2461,7 +2461,7 @@ static void am_begin(Engine &E, AmRun &R, const pscfg_am_param &prm)
         double *part = E.part((size_t)nct * nj);
         k_partial_sum<double><<<dim3(nct, nj), 256, 0, E.st>>>(dwp, E.nr, part);
         E.launched();
-        k_final_sum<<<(unsigned)((nj + 127) / 128), 128, 0, E.st>>>(part, nct, (double)E.nr, E.d_small, nj);
+        k_final_sum<<<(unsigned)((nj + 3) / 4), 128, 0, E.st>>>(part, nct, (double)E.nr, E.d_small, nj);
         E.launched();
         k_omega_uniform<<<dim3(red_ctas(E.nr, ninst), ninst), 256, 0, E.st>>>(duj, E.nr);
         E.launched();
@@ -2545,7 +2545,7 @@ static int am_iterate(Engine &E, AmRun &R, int iters)
         double *dpart = mpart + (size_t)nct * na;
         k_am_dev<<<dim3(nct, na), 256, 0, E.st>>>(daj, E.nr, part);
         E.launched();
-        k_final_sum<<<(unsigned)((na * PSCFG_MAXM + 127) / 128), 128, 0, E.st>>>(part, nct, (double)E.nr, E.d_small,
+        k_final_sum<<<(unsigned)((na * PSCFG_MAXM + 3) / 4), 128, 0, E.st>>>(part, nct, (double)E.nr, E.d_small,
                                                                                   na * PSCFG_MAXM);
         E.launched();
         std::vector<AmFix> fx;
@@ -2583,7 +2583,7 @@ static int am_iterate(Engine &E, AmRun &R, int iters)
         k_am_dots<<<dim3(nct, na), 256, 0, E.st>>>(ddot, dpart);
         E.launched();
         double *dres = E.d_small + (size_t)na * (PSCFG_MAXM + 1);
-        k_final_sum<<<(unsigned)((na * (PSCFG_MAXH + 1) + 127) / 128), 128, 0, E.st>>>(dpart, nct, 1.0, dres,
+        k_final_sum<<<(unsigned)((na * (PSCFG_MAXH + 1) + 3) / 4), 128, 0, E.st>>>(dpart, nct, 1.0, dres,
                                                                                        na * (PSCFG_MAXH + 1));
         E.launched();
         double *dstat = dres + (size_t)na * (PSCFG_MAXH + 1);
@@ -2915,7 +2915,7 @@ static void amg_iteration(Engine &E, AmRun &R, const std::vector<int> &act)
     double *dpart = mpart + (size_t)nct * na;
     k_am_dev<<<dim3(nct, na), 256, 0, E.st>>>(R.g_aj, E.nr, part);
     E.launched();
-    k_final_sum<<<(unsigned)((na * PSCFG_MAXM + 127) / 128), 128, 0, E.st>>>(part, nct, (double)E.nr, E.d_small,
+    k_final_sum<<<(unsigned)((na * PSCFG_MAXM + 3) / 4), 128, 0, E.st>>>(part, nct, (double)E.nr, E.d_small,
                                                                               na * PSCFG_MAXM);
     E.launched();
     k_am_fix<<<dim3(nct, na), 256, 0, E.st>>>(R.g_fx, E.nr, mpart);
@@ -2926,7 +2926,7 @@ static void amg_iteration(Engine &E, AmRun &R, const std::vector<int> &act)
     k_am_dots<<<dim3(nct, na), 256, 0, E.st>>>(R.g_dots, dpart);
     E.launched();
     double *dres = E.d_small + (size_t)na * (PSCFG_MAXM + 1);
-    k_final_sum<<<(unsigned)((na * (PSCFG_MAXH + 1) + 127) / 128), 128, 0, E.st>>>(dpart, nct, 1.0, dres,
+    k_final_sum<<<(unsigned)((na * (PSCFG_MAXH + 1) + 3) / 4), 128, 0, E.st>>>(dpart, nct, 1.0, dres,
                                                                                    na * (PSCFG_MAXH + 1));
     E.launched();
     double *dstat = dres + (size_t)na * (PSCFG_MAXH + 1);
@@ -2946,7 +2946,7 @@ static void amg_iteration(Engine &E, AmRun &R, const std::vector<int> &act)
     k_am_mix<<<dim3(nct, na), 256, 0, E.st>>>(R.g_mix);
     E.launched();
     if (R.g_maxorb > 0) {
-        dim3 grid((unsigned)std::max(1, std::min((R.g_maxorb + 127) / 128, 256)), (unsigned)na);
+        dim3 grid((unsigned)std::max(1, std::min((R.g_maxorb * SYM_LANES + 127) / 128, 1024)), (unsigned)na);
         k_symmetrize<<<grid, 128, 0, E.st>>>(R.g_sym, E.nr);
         E.launched();
     }
@@ -3297,7 +3297,7 @@ static void adjoint_impl(Engine &E, const std::vector<int> &act, const std::vect
             double *part = E.part((size_t)nct * os.size());
             k_adj_overlap<T><<<dim3(nct, (unsigned)os.size()), 256, 0, E.st>>>(dov, nr, part);
             E.launched();
-            k_final_sum<<<(unsigned)((os.size() + 127) / 128), 128, 0, E.st>>>(part, nct, 1.0, E.d_small, (int)os.size());
+            k_final_sum<<<(unsigned)((os.size() + 3) / 4), 128, 0, E.st>>>(part, nct, 1.0, E.d_small, (int)os.size());
             E.launched();
             std::vector<double> h(os.size());
             CK(cudaMemcpyAsync(h.data(), E.d_small, sizeof(double) * os.size(), cudaMemcpyDeviceToHost, E.st));
@@ -3311,7 +3311,7 @@ static void adjoint_impl(Engine &E, const std::vector<int> &act, const std::vect
         double *part = E.part((size_t)nct * ov.size());
         k_adj_overlap<T><<<dim3(nct, (unsigned)ov.size()), 256, 0, E.st>>>(dov, nr, part);
         E.launched();
-        k_final_sum<<<(unsigned)((ov.size() + 127) / 128), 128, 0, E.st>>>(part, nct, 1.0, E.d_small, (int)ov.size());
+        k_final_sum<<<(unsigned)((ov.size() + 3) / 4), 128, 0, E.st>>>(part, nct, 1.0, E.d_small, (int)ov.size());
         E.launched();
         CK(cudaMemcpyAsync(Sc.data(), E.d_small, sizeof(double) * ov.size(), cudaMemcpyDeviceToHost, E.st));
         CK(cudaStreamSynchronize(E.st));

@@ -357,24 +357,31 @@ __global__ void k_partial_sum(const T *const *ptrs, long n, double *part)
     if (threadIdx.x == 0) part[(long)blockIdx.y * gridDim.x + blockIdx.x] = s;
 }
 
-// Fixed-order final reduction of npart partials per job: out[j] = sum/div.
+// Fixed-order final reduction of npart partials per job, one warp per job:
+// out[j] = sum/div.  (One thread per job added 592 partials in 20 us.)
+__device__ __forceinline__ double final_sum(const double *part, int npart, int j)
+{
+    double s = 0.0;
+    for (int i = threadIdx.x & 31; i < npart; i += 32) s += part[(long)j * npart + i];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    return s;   // valid in lane 0
+}
+
 static __global__ void k_final_sum(const double *part, int npart, double div, double *out, int njobs)
 {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= njobs) return;
-    double s = 0.0;
-    for (int i = 0; i < npart; i++) s += part[(long)j * npart + i];
-    out[j] = s / div;
+    const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (j >= njobs) return;   // whole warps
+    const double s = final_sum(part, npart, j);
+    if ((threadIdx.x & 31) == 0) out[j] = s / div;
 }
 
 // Same, writing job j's result to *outs[j].
 static __global__ void k_final_sum_ptr(const double *part, int npart, double div, double *const *outs, int njobs)
 {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (j >= njobs) return;
-    double s = 0.0;
-    for (int i = 0; i < npart; i++) s += part[(long)j * npart + i];
-    *outs[j] = s / div;
+    const double s = final_sum(part, npart, j);
+    if ((threadIdx.x & 31) == 0) *outs[j] = s / div;
 }
 
 // Simpson contour integral for one (instance, chain): rho of each block,

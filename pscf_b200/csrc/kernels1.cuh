@@ -82,12 +82,19 @@ __global__ void __launch_bounds__(4 * NMAX) k1_sweep_dense(const SweepField<T> *
             const int i = row < n ? row : 0;
 #pragma unroll
             for (int j = 0; j < 2 * J; j++) a[j] = 0.0;
+            // c2[m - col] of an odd column is what the even one before it had
+            // at m - 1: one shared-memory read for two multiply-adds
+            double co[J];
+#pragma unroll
+            for (int j = 0; j < J; j++) co[j] = c2[max(n - 1 - (8 * j + 2 * l), 0)];
             for (int m = 0; m < n; m++) {
                 const double x = c2[i - m + n] * e1[m];
 #pragma unroll
-                for (int j = 0; j < 2 * J; j++) {
-                    const int col = min(8 * (j >> 1) + 2 * l + (j & 1), n - 1);
-                    a[j] += x * c2[m - col + n];
+                for (int j = 0; j < J; j++) {
+                    const double ce = c2[m - min(8 * j + 2 * l, n - 1) + n];
+                    a[2 * j] += x * ce;
+                    a[2 * j + 1] += x * co[j];
+                    co[j] = ce;
                 }
             }
 #pragma unroll
