@@ -1255,7 +1255,6 @@ static void sweep_steps(Engine &E, const SweepField<T> *dfl, int nf, int t0, int
 {
     const PlaneGeom &g = E.geom();
     const int ns_max = t1;
-    if (E.dim == 2 && !E.no_fixed_kernels && E.launched_n(rx2_sweep<T>(E.rx, E.st, dfl, nf, t0, t1))) return;
     if (E.dim == 1 && !E.no_fixed_kernels && E.nr <= 128) {
         // the step as a dense matrix held in registers; 128 points are the
         // most whose matrix (128 KB) one CTA's registers hold
@@ -1270,6 +1269,7 @@ static void sweep_steps(Engine &E, const SweepField<T> *dfl, int nf, int t0, int
     if (E.dim <= 2) {
         size_t sm = 2 * (size_t)g.n2 * g.LS * sizeof(cx<T>) + 2 * (size_t)E.nr * sizeof(T);
         if (sm > 227 * 1024) throw Err(PSCFG_EINVAL, "grid too large for the single-CTA plane step");
+        if (E.dim == 2 && !E.no_fixed_kernels && E.launched_n(rx2_sweep<T>(E.rx, E.st, dfl, nf, t0, t1))) return;
         CK(allow_dyn_smem((const void *)k_sweep_plane<T>));
         // one CTA per field: a sweep of few fields is bound by the latency of
         // its FFT phases, which more warps hide (64 x 64 with this kernel,
@@ -1995,22 +1995,22 @@ static void slice_dots(Engine &E, const std::vector<StressJob<T>> &jobs)
         for (auto &j : jobs) maxs = std::max(maxs, j.nslices);
         if (slice_dots_r<T>(E, dj, (int)jobs.size(), maxs)) return;
     }
-    if (rx3_applies<T>(E)) {
+    // (the run-time shaped kernels' limits stay the limits of the stress)
+    if (rx3_applies<T>(E) && 2 * (size_t)g.n2 * g.LS * sizeof(cx<T>) <= 227 * 1024 &&
+        4 * (size_t)g.n3 * Z_TILE * sizeof(cx<T>) <= 227 * 1024) {
         int maxs = 0;
         for (auto &j : jobs) maxs = std::max(maxs, j.nslices);
         if (slice_dots_v<T>(E, dj, (int)jobs.size(), maxs)) return;
     }
     size_t off = ((jobs.size() * sizeof(StressJob<T>) + 255) / 256) * 256;
-    if (E.dim == 2 && !E.no_fixed_kernels) {
-        int maxs = 0;
-        for (auto &j : jobs) maxs = std::max(maxs, j.nslices);
-        if (jobs.size() <= 65535 && E.launched_n(rx2_stress<T>(E.rx, E.st, dj, (int)jobs.size(), maxs))) return;
-    }
     if (E.dim <= 2) {
         int maxs = 0;
         for (auto &j : jobs) maxs = std::max(maxs, j.nslices);
         size_t sm = 4 * (size_t)g.n2 * g.LS * sizeof(cx<T>);
         if (sm > 227 * 1024) throw Err(PSCFG_EINVAL, "grid too large for the plane stress kernel");
+        if (E.dim == 2 && !E.no_fixed_kernels && jobs.size() <= 65535 &&
+            E.launched_n(rx2_stress<T>(E.rx, E.st, dj, (int)jobs.size(), maxs)))
+            return;
         CK(allow_dyn_smem((const void *)k2_stress_slices<T>));
         int threads = (int)std::min<long>(256, std::max<long>(32, ((E.nr / 2 + 31) / 32) * 32));
         k2_stress_slices<T><<<dim3(maxs, (unsigned)jobs.size()), threads, sm, E.st>>>(dj, g);
@@ -3145,7 +3145,6 @@ static void run_single_steps(Engine &E, const SweepField<T> *dfl, int nf)
 {
     const PlaneGeom &g = E.geom();
     const long nr = E.nr;
-    if (E.dim == 2 && !E.no_fixed_kernels && E.launched_n(rx2_sweep<T>(E.rx, E.st, dfl, nf, 0, 1))) return;
     if (rx3_applies<T>(E)) {
         E.launched_n(rx3_first<T>(E.rx, E.st, dfl, nf, 0));
         E.launched_n(rx3_step<T>(E.rx, E.st, dfl, nf, 0));
@@ -3153,6 +3152,7 @@ static void run_single_steps(Engine &E, const SweepField<T> *dfl, int nf)
     }
     if (E.dim <= 2) {
         size_t sm = 2 * (size_t)g.n2 * g.LS * sizeof(cx<T>) + 2 * (size_t)nr * sizeof(T);
+        if (E.dim == 2 && !E.no_fixed_kernels && sm <= 227 * 1024 && E.launched_n(rx2_sweep<T>(E.rx, E.st, dfl, nf, 0, 1))) return;
         CK(allow_dyn_smem((const void *)k_sweep_plane<T>));
         int threads = (int)std::min<long>(256, std::max<long>(32, ((nr / 2 + 31) / 32) * 32));
         k_sweep_plane<T><<<nf, threads, sm, E.st>>>(dfl, g, 0, 1);
