@@ -134,6 +134,14 @@ template <typename T> __host__ __device__ __forceinline__ constexpr int rx_slot(
 {
     return Q1 * k1 + (k2 + rx_rot<T>(Q1, k1)) % Q1;
 }
+// Line of the row passes' l-th group of Q1 = 8 items.  An 8-byte half warp
+// holds two groups, whose lines must lie 8 units apart on the 16 bank pairs:
+// lines j and j + 8 at an odd stride (fixed shapes: whole blocks of 16 lines).
+template <typename T, typename SH> __device__ __forceinline__ int rx_line(int l)
+{
+    if constexpr (SH::FIXED && sizeof(T) == 4) return (l & ~15) | ((l & 1) << 3) | ((l >> 1) & 7);
+    else return l;
+}
 // line stride in complex values: n1 slots, two spare ones, odd
 __host__ __device__ __forceinline__ constexpr int rx_stride(int n1) { return (n1 + 2) | 1; }
 
@@ -893,7 +901,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NT, MB)
 template <int P, typename T, typename SH>
 __device__ __forceinline__ void rp_load(const SH &sh, const RxMem<T, SH> &m, int w, int line0, const T *src)
 {
-    const int l = sh.dQ1.div(w), r = w - sh.Q1 * l, y0 = l + sh.Q2 * sh.dQ2.div(l);   // r2 + 2 j Q2
+    const int lw = sh.dQ1.div(w), r = w - sh.Q1 * lw, l = rx_line<T, SH>(lw), y0 = l + sh.Q2 * sh.dQ2.div(l);   // r2 + 2 j Q2
     const bool two = y0 + sh.Q2 < sh.n2;
     const T *a = src + y0 * sh.n1 + r, *b = a + sh.Q2 * sh.n1;
     cx<T> v[P];
@@ -1022,7 +1030,7 @@ __global__ void __launch_bounds__(NT, MB)
     auto go = [&](auto pc) {
         constexpr int P = decltype(pc)::value;
         for (int w = threadIdx.x; w < np * sh.n2 * sh.Q1; w += blockDim.x) {
-            const int l = sh.dQ1.div(w), r = w - sh.Q1 * l;
+            const int lw = sh.dQ1.div(w), r = w - sh.Q1 * lw, l = rx_line<T, SH>(lw);
             cx<T> v[P];
 #pragma unroll
             for (int i = 0; i < P; i++) {
@@ -1075,7 +1083,7 @@ __global__ void __launch_bounds__(NT, MB)
     auto go = [&](auto pc) {
         constexpr int P = decltype(pc)::value;
         for (int w = threadIdx.x; w < np * npair * sh.Q1; w += blockDim.x) {
-            const int l = sh.dQ1.div(w), r = w - sh.Q1 * l;
+            const int lw = sh.dQ1.div(w), r = w - sh.Q1 * lw, l = rx_line<T, SH>(lw);
             const int pl = dpair.div(l), lp = l - npair * pl, j = sh.dQ2.div(lp);
             const int y0 = lp + sh.Q2 * j;   // r2 + 2 j Q2
             const bool two = y0 + sh.Q2 < sh.n2;
@@ -1153,7 +1161,7 @@ __global__ void __launch_bounds__(NT, MB)
     auto go = [&](auto pc) {
         constexpr int P = decltype(pc)::value;
         for (int w = threadIdx.x; w < np * sh.n2 * sh.Q1; w += blockDim.x) {
-            const int l = sh.dQ1.div(w), r = w - sh.Q1 * l, x0 = l * sh.n1 + r;
+            const int lw = sh.dQ1.div(w), r = w - sh.Q1 * lw, l = rx_line<T, SH>(lw), x0 = l * sh.n1 + r;
             C v[P];
             T e[P], en[P];
             // (ahead of the stores to out, which the compiler must assume to
