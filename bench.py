@@ -413,8 +413,8 @@ def run_ours(args, rank, world, local_rank):
         return
     s0 = wl.systems[0]
     peak, peak_kind = measured_peaks()
-    kernel = ("MDE step: k3p_final_fwd + k3p_zconv x2 + k3p_mid (kernels3p.cuh, 64x128x224)" if args.config == "c5"
-              else "MDE step: k3r_final_fwd + k3s_zconv x2 + k3r_inv_mid (kernels3c.cuh, 32^3)")
+    kernel = ("MDE step: k3v_final + k3v_zconv x2 + k3v_mid (plane_rx.cuh, 64x128x224)" if args.config == "c5"
+              else "MDE step: k3v_final + k3v_zconv x2 + k3v_mid (plane_rx.cuh, 32^3)")
     cpu = None
     if world == 1 and not args.no_cpu:
         nthreads = os.cpu_count() or 1
@@ -582,7 +582,7 @@ def c2_leg(args, rank, world, barrier, dev, local_rank):
     out = {"workload": WORKLOAD_C2, "batch_per_gpu": 64, "value": total / elapsed, "unit": "MDE steps/s",
            "ms_per_step": 1e3 * elapsed / steps, "steps": steps,
            "roofline": roofline(wl.systems[0], prof, nsteps, peak, peak_kind, 8,
-                                "MDE step: k3r_final_fwd + k3s_zconv x2 + k3r_inv_mid (kernels3c.cuh, 32^3)"),
+                                "MDE step: k3v_final + k3v_zconv x2 + k3v_mid (plane_rx.cuh, 32^3)"),
            "sweep_steps_per_s_fp64": nsteps / (prof["sweep_ms"] / 1e3),
            "planes_per_cta": e.sweep_planes(2 * len(wl.systems))}
     if not args.no_solve:

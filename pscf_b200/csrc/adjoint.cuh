@@ -22,6 +22,7 @@ struct AdjPoint {
     // step intermediates of the adjoint state (lam) and of the stored slice (q)
     const void *lam, *p1l, *hl, *p2l;
     const void *q, *p1q, *hq, *p2q;
+    const void *qn;             // p2q null: the stored slice after q, P2 q = (3 qn + P1 q) / 4
     const void *eo1;            // block table exp(-w ds/2)
     double ds;
     double *grad;               // dL/domega of the block's monomer (accumulated)
@@ -39,13 +40,14 @@ __global__ void k_adj_point(const AdjPoint *jobs, long nr)
     const AdjPoint &J = jobs[blockIdx.y];
     const T *lam = (const T *)J.lam, *p1l = (const T *)J.p1l, *hl = (const T *)J.hl, *p2l = (const T *)J.p2l;
     const T *q = (const T *)J.q, *p1q = (const T *)J.p1q, *hq = (const T *)J.hq, *p2q = (const T *)J.p2q;
-    const T *eo1 = (const T *)J.eo1, *other = (const T *)J.other;
+    const T *eo1 = (const T *)J.eo1, *other = (const T *)J.other, *qn = (const T *)J.qn;
     T *ln = (T *)J.lam_new;
     const double ds = J.ds;
     for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < nr; r += (long)gridDim.x * blockDim.x) {
         const double l = lam[r], x = q[r];
         const double d1 = -(ds / 2.0) * (l * (double)p1q[r] + x * (double)p1l[r]);
-        const double d2 = -(ds / 4.0) * (l * (double)p2q[r] + x * (double)p2l[r]) -
+        const double p2 = p2q ? (double)p2q[r] : (3.0 * (double)qn[r] + (double)p1q[r]) / 4.0;
+        const double d2 = -(ds / 4.0) * (l * p2 + x * (double)p2l[r]) -
                           (ds / 2.0) * (double)hl[r] * (double)hq[r] / (double)eo1[r];
         J.grad[r] += (4.0 * d2 - d1) / 3.0;
         double dir = 0.0;

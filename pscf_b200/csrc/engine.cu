@@ -3358,8 +3358,13 @@ static void adjoint_impl(Engine &E, const std::vector<int> &act, const std::vect
         if (!E.ckpt) return (const T *)(which == 0 ? I.qf[c] : I.qr[c]) + (long)sl * nr;
         return (const T *)(which == 0 ? I.segA[c] : I.segB[c]) + (long)(sl - j_seg * E.ckK) * nr;
     };
+    // The stored slice's second half step need not be made again: the slice
+    // after it holds the step's result.  Its fields then take 3 launches
+    // (k3v_half) beside lambda's 5 on a second stream (not with the cell
+    // derivative, whose pairs are formed from P2 q itself).
+    const bool half = rx3_applies<T>(E) && !want_cell;
     auto adj_step = [&](int t, const std::vector<size_t> &sel) {
-        std::vector<SweepField<T>> fl;
+        std::vector<SweepField<T>> fl, flq;
         std::vector<AdjPoint> pts;
         for (size_t si : sel) {
             auto &S = sw[si];
@@ -3403,7 +3408,7 @@ static void adjoint_impl(Engine &E, const std::vector<int> &act, const std::vect
                 F.out = S.dummy[f];
                 F.h_out = S.h[f];
                 F.q2_out = S.p2[f];
-                fl.push_back(F);
+                (half && f == 1 ? flq : fl).push_back(F);
             }
             AdjPoint a;
             std::memset(&a, 0, sizeof(a));
@@ -3414,7 +3419,8 @@ static void adjoint_impl(Engine &E, const std::vector<int> &act, const std::vect
             a.q = qsrc;
             a.p1q = S.p1[1];
             a.hq = S.h[1];
-            a.p2q = S.p2[1];
+            a.p2q = half ? nullptr : S.p2[1];
+            a.qn = S.d == 0 ? slice(I, S.c, 0, qslice + 1) : slice(I, S.c, 1, qslice - 1);
             a.eo1 = I.eo1[S.c][blk];
             a.ds = I.bds[S.c][blk];
             a.grad = S.gbuf + (long)I.sys.block_monomer[S.c][blk] * nr;
@@ -3425,10 +3431,22 @@ static void adjoint_impl(Engine &E, const std::vector<int> &act, const std::vect
             a.M = E.M;
             pts.push_back(a);
         }
+        const int nl = (int)fl.size();
+        fl.insert(fl.end(), flq.begin(), flq.end());
         SweepField<T> *dfl = E.upload(fl, 0);
         size_t o2 = ((fl.size() * sizeof(SweepField<T>) + 255) / 256) * 256;
         AdjPoint *dpt = E.upload(pts, o2);
-        run_single_steps<T>(E, dfl, (int)fl.size());
+        if (half && nl > 0) {
+            CK(cudaEventRecord(E.ev_fork, E.st));
+            CK(cudaStreamWaitEvent(E.st2, E.ev_fork, 0));
+            E.launched_n(rx3_first<T>(E.rx, E.st2, dfl + nl, (int)flq.size(), 0));
+            E.launched_n(rx3_half<T>(E.rx, E.st2, dfl + nl, (int)flq.size()));
+            CK(cudaEventRecord(E.ev_join, E.st2));
+            run_single_steps<T>(E, dfl, nl);
+            CK(cudaStreamWaitEvent(E.st, E.ev_join, 0));
+        } else {
+            run_single_steps<T>(E, dfl, (int)fl.size());
+        }
         k_adj_point<T><<<dim3((unsigned)std::min<long>((nr + 255) / 256, 256), (unsigned)pts.size()), 256, 0, E.st>>>(dpt, nr);
         E.launched();
         if (want_cell) {

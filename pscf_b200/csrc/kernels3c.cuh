@@ -938,11 +938,14 @@ __global__ void k3_stress_sum_b(const StressJob<T> *jobs, int s0, int cs, int nt
     const int job = blockIdx.y;
     const StressJob<T> &J = jobs[job];
     const int s = s0 + blockIdx.x;
-    if (s >= J.nslices || threadIdx.x >= J.ncp) return;
-    const int b = threadIdx.x;
-    double acc = 0.0;
-    for (int t = 0; t < ntiles; t++) acc += part[(((long)job * cs + blockIdx.x) * ntiles + t) * PSCFG_MAXCP + b];
-    J.inc[(long)s * PSCFG_MAXCP + b] = acc;
+    if (s >= J.nslices) return;
+    // one warp: lanes over the tiles (a thread per sum took 37 us for 528)
+    for (int b = 0; b < J.ncp; b++) {
+        double acc = 0.0;
+        for (int t = threadIdx.x; t < ntiles; t += 32) acc += part[(((long)job * cs + blockIdx.x) * ntiles + t) * PSCFG_MAXCP + b];
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+        if (threadIdx.x == 0) J.inc[(long)s * PSCFG_MAXCP + b] = acc;
+    }
 }
 
 // Pass 2: z-forward of both spectra on TC columns and the weighted dot

@@ -1189,6 +1189,56 @@ __global__ void __launch_bounds__(NT, MB)
     Rx3<T, SH>::fwd_fp(sh, m, np, f.S2 + so, f.S1 + so);
 }
 
+// After k3v_fwd and k3v_zconv on S1 and S2: q1 = eo1 Fxy^-1[S1] / N and
+// h = eo1 Fxy^-1[S2] / N alone (the adjoint's steps of stored slices, whose
+// second half step follows from the next slice).  ns = 1 fields, t = 0.
+template <typename T, typename SH, int NT, int MB>
+__global__ void __launch_bounds__(NT, MB) k3v_half(const SweepField<T> *fields, SH sh, RxTables tb, int n3, int ppc)
+{
+    using X = Rx<T, SH>;
+    using C = cx<T>;
+    const SweepField<T> &f = fields[blockIdx.y];
+    const int z0 = blockIdx.x * ppc, np = min(ppc, n3 - z0), npl = sh.n1 * sh.n2;
+    const long po = (long)z0 * npl, so = (long)z0 * sh.n2 * sh.n1h;
+    const C *sa = f.S2 + so, *sb = f.S1 + so;
+    const RxMem<T, SH> m(sh, tb, ppc * sh.n2);
+    const T rn = (T)(2.0 * npl * n3), rr = (T)(1.0 / (2.0 * npl * n3));
+    const T *e2 = f.eo2[0] + po;
+    T *q1 = f.q1 + po, *h = f.h_out + po;
+    if (!SH::FIXED) __syncthreads();
+    X::template cols2<true, 1>(sh, m.buf, np, sh.n2, m.ct, [&](auto qc, int c, int, int ab, int pl, int k1, C *s, C *v) {
+        constexpr int Q = decltype(qc)::value;
+        const C *d = (ab ? sb : sa) + (long)(pl * sh.n2 + k1) * sh.n1h + c;
+#pragma unroll
+        for (int k = 0; k < Q; k++) v[k] = d[(long)sh.n1h * sh.P2 * k];
+        Dft<Q, 1, T>::run(v);
+#pragma unroll
+        for (int n = 0; n < Q; n++) s[n * sh.LS] = v[n];
+    });
+    __syncthreads();
+    X::template cols_inv1<true, 1>(sh, m.buf, np, sh.n2, m.ct, m.tw2);
+    __syncthreads();
+    X::template rows2<1>(sh, m.buf, np * sh.n2, RDiv::of(np * sh.n2), [](int l) { return l; });
+    __syncthreads();
+    auto go = [&](auto pc) {
+        constexpr int P = decltype(pc)::value;
+        for (int w = threadIdx.x; w < np * sh.n2 * sh.Q1; w += blockDim.x) {
+            const int lw = sh.dQ1.div(w), r = w - sh.Q1 * lw, l = rx_line<T, SH>(lw), x0 = l * sh.n1 + r;
+            C v[P];
+            T e[P];
+#pragma unroll
+            for (int i = 0; i < P; i++) e[i] = e2[x0 + sh.Q1 * i];
+            X::template row_inv1<P>(sh, m.buf + l * sh.LS, r, v, m.tw1);
+#pragma unroll
+            for (int i = 0; i < P; i++) {
+                h[x0 + sh.Q1 * i] = div_by(e[i] * e[i] * v[i].x, rn, rr);
+                q1[x0 + sh.Q1 * i] = div_by(e[i] * e[i] * v[i].y, rn, rr);
+            }
+        }
+    };
+    RX_P(SH, P1, go);
+}
+
 // x-y transform of slices s0 .. s0 + cs of qf and qr of every job (RP
 // planes, see k2x_stress); spectra at ((job cs + slice) 2 + which) nk.
 // grid = (planes / ppc, cs, 2 njobs).

@@ -28,6 +28,7 @@ template <typename T> int rx2_stress(const RxPlan &p, cudaStream_t st, const Str
 template <typename T> bool rx3_fits(const RxPlan &p);
 template <typename T> int rx3_planes(const RxPlan &p, int nf);   // planes per CTA of the x-y kernels
 template <typename T> int rx3_first(const RxPlan &p, cudaStream_t st, const SweepField<T> *f, int nf, int t);
+template <typename T> int rx3_half(const RxPlan &p, cudaStream_t st, const SweepField<T> *f, int nf);   // k3v_half, and the z pass before it
 template <typename T> int rx3_step(const RxPlan &p, cudaStream_t st, const SweepField<T> *f, int nf, int t);
 template <typename T> int rx3_stress_tiles(const RxPlan &p);
 template <typename T>

@@ -193,6 +193,20 @@ template <typename T> static int zconv(const RxPlan &p, cudaStream_t st, const S
     });
 }
 
+template <typename T> int rx3_half(const RxPlan &p, cudaStream_t st, const SweepField<T> *f, int nf)
+{
+    if (!rx3_fits<T>(p)) return 0;
+    if (zconv<T>(p, st, f, nf, 0, 3) < 0) return -1;
+    const int rc = with_plane<T>(p, rx3_ctas<T>(p, nf), [&](auto sh, auto nt, auto mb, auto, auto) {
+        const int ppc = rx3_planes<T>(p, nf);
+        auto *k = k3v_half<T, decltype(sh), decltype(nt)::value, decltype(mb)::value>;
+        RX_LAUNCH(k, dim3((p.n3 + ppc - 1) / ppc, nf), fp_threads<T>(p.sh, ppc, decltype(nt)::value), fp_bytes<T>(p.sh, ppc),
+                  st, f, sh, p.tb[prec_of<T>()], p.n3, ppc);
+        return 1;
+    });
+    return rc < 0 ? -1 : 2;
+}
+
 template <typename T> int rx3_step(const RxPlan &p, cudaStream_t st, const SweepField<T> *f, int nf, int t)
 {
     if (!rx3_fits<T>(p)) return 0;
@@ -259,6 +273,7 @@ int rx3_stress(const RxPlan &p, cudaStream_t st, const StressJob<T> *jobs, int n
     template int rx3_planes<T>(const RxPlan &, int);                                                                 \
     template bool rx3_fits<T>(const RxPlan &);                                                                       \
     template int rx3_first<T>(const RxPlan &, cudaStream_t, const SweepField<T> *, int, int);                        \
+    template int rx3_half<T>(const RxPlan &, cudaStream_t, const SweepField<T> *, int);                              \
     template int rx3_step<T>(const RxPlan &, cudaStream_t, const SweepField<T> *, int, int);                         \
     template int rx3_stress_tiles<T>(const RxPlan &);                                                                \
     template int rx3_stress<T>(const RxPlan &, cudaStream_t, const StressJob<T> *, int, int, int, int, cx<T> *, double *);
