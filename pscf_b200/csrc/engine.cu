@@ -942,10 +942,11 @@ static bool rx3_applies(const Engine &E)
 // A whole 3-D sweep with the plane_rx.cuh kernels.  The fields of a group
 // run as two independent kernel chains on two streams, so that each launch's
 // last, partly empty wave overlaps the other chain's work; a batch whose
-// step scratch (both spectra, the block's table, two slices) overflows the L2 goes in groups
-// that fit it, each group through the whole contour (32^3 x 64 instances:
-// sweep 21.1 ms in groups of 32 or 64 fields, 23.1 at once, 25.5 in groups
-// of 16, whose launches no longer fill the GPU).
+// step scratch (both spectra, the block's table, two slices) overflows the
+// L2 goes in groups that fit it, each group through the whole contour (32^3
+// x 64 instances, density + stress when this was chosen: 21.1 ms in groups of
+// 32 or 64 fields, 23.1 at once, 25.5 in groups of 16, whose launches no
+// longer fill the GPU).
 template <typename T>
 static bool sweep3v(Engine &E, const SweepField<T> *dfl, int nf, int ns_max, int t0 = 0)
 {

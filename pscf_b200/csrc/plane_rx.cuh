@@ -152,7 +152,7 @@ struct RxShape {
     static constexpr bool FIXED = false;
     static constexpr int PM = 10, QM = 16;
     int n1, n2, n1h, nc, P1, Q1, P2, Q2, HP, LS;   // nc: columns without kx = n1/2
-    RDiv dQ1, dn1h, dnc, dQ2, dP2, dn2;
+    RDiv dQ1, dn1h, dnc, dQ2, dP2;
 };
 struct RxShape10 : RxShape {
     static constexpr int PM = 8, QM = 10;
@@ -167,7 +167,6 @@ template <int N1, int N2, int P1_, int P2_> struct RxFixed {
     SDiv<(N1 + 1) / 2> dnc;
     SDiv<N2 / P2_> dQ2;
     SDiv<P2_> dP2;
-    SDiv<N2> dn2;
 };
 
 // Column c of a fixed shape (even Q1: every k1 group holds Q1 / 2 columns, kx

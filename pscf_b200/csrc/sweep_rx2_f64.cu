@@ -43,7 +43,6 @@ bool rx_shape(int dim, const int n[3], RxPlan &p, RxCol *cols, bool f32)
     s.dnc = RDiv::of(s.nc);
     s.dQ2 = RDiv::of(s.Q2);
     s.dP2 = RDiv::of(s.P2);
-    s.dn2 = RDiv::of(s.n2);
     int c = 0;
     auto slot = [&](int kx) {
         return f32 ? rx_slot<float>(s.Q1, kx % s.P1, kx / s.P1) : rx_slot<double>(s.Q1, kx % s.P1, kx / s.P1);
