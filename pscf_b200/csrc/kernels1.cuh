@@ -28,8 +28,8 @@ namespace pscfg {
 // row of a warp).  All arithmetic in FP64, also for FP32 slabs.
 // Bound: the serial chain of a step (shared-memory read, NMAX/16 dependent
 // multiply-adds, two shuffles, write, barrier).  64 points, 100 steps of a
-// diblock: 74 us, of which about half is the two blocks' matrices, against
-// 1132 us with k_sweep_plane; 192 fields: 108 us against 1166.
+// diblock: 70 us, the two blocks' matrices included, against 1132 us with
+// k_sweep_plane; 192 fields: 97 us against 1166.
 // grid = nfields, 4 NMAX threads.
 template <typename T, int NMAX>
 __global__ void __launch_bounds__(4 * NMAX) k1_sweep_dense(const SweepField<T> *fields, int n, int t0, int t1,
