@@ -1128,7 +1128,7 @@ static bool step3_fixed(Engine &E, const SweepField<T> *dfl, int nf, int t)
 }
 
 template <typename T>
-static void sweep_steps(Engine &E, const SweepField<T> *dfl, int nf, int t0, int t1);
+static void sweep_steps(Engine &E, const std::vector<SweepField<T>> &fl, const SweepField<T> *dfl, int t0, int t1);
 
 template <typename T>
 static void run_sweeps(Engine &E, const std::vector<int> &act)
@@ -1246,19 +1246,35 @@ static void run_sweeps(Engine &E, const std::vector<int> &act)
         k_init_ends<T><<<g2, 256, 0, E.st>>>(dfl, E.nr);
         E.launched();
     }
-    sweep_steps<T>(E, dfl, (int)fl.size(), 0, ns_max);
+    sweep_steps<T>(E, fl, dfl, 0, ns_max);
 }
 
-// Steps t in [t0, t1) of every field at dfl (t counts the steps of each
-// field's own sweep, step_slices), on whichever kernels the grid has.
+// Whether steps [t0, t1) of these 1-D fields take the dense step.  128
+// points are the most whose matrix (128 KB) one CTA's registers hold.
 template <typename T>
-static void sweep_steps(Engine &E, const SweepField<T> *dfl, int nf, int t0, int t1)
+static bool dense1d_applies(const Engine &E, const std::vector<SweepField<T>> &fl, int t0, int t1)
+{
+    if (E.dim != 1 || E.no_fixed_kernels || E.nr > 128) return false;
+    long steps = 0, blocks = 0;
+    for (const auto &f : fl) {
+        // the steps as slices [lo, hi] (step_slices), and the blocks they meet
+        const int te = std::min(t1, f.ns), lo = f.dir > 0 ? t0 : f.ns - te, hi = f.dir > 0 ? te : f.ns - t0;
+        if (hi <= lo) continue;
+        steps += hi - lo;
+        for (int b = 0; b < f.nblk; b++) blocks += std::max(lo, f.bgn[b]) < std::min(hi, f.bgn[b + 1]);
+    }
+    return k1_dense_pays((int)E.nr, (int)fl.size(), steps, blocks);
+}
+
+// Steps t in [t0, t1) of every field at dfl, the device copy of fl (t counts
+// the steps of each field's own sweep, step_slices), on whichever kernels the
+// grid has.
+template <typename T>
+static void sweep_steps(Engine &E, const std::vector<SweepField<T>> &fl, const SweepField<T> *dfl, int t0, int t1)
 {
     const PlaneGeom &g = E.geom();
-    const int ns_max = t1;
-    if (E.dim == 1 && !E.no_fixed_kernels && E.nr <= 128) {
-        // the step as a dense matrix held in registers; 128 points are the
-        // most whose matrix (128 KB) one CTA's registers hold
+    const int ns_max = t1, nf = (int)fl.size();
+    if (dense1d_applies<T>(E, fl, t0, t1)) {
         const int n = E.n[0];
         const cx<double> *tw = (const cx<double> *)E.g64.rtw;
         if (n <= 32) k1_sweep_dense<T, 32><<<nf, 128, 0, E.st>>>(dfl, n, t0, t1, tw);
@@ -1612,7 +1628,7 @@ static void ckpt_segment(Engine &E, const std::vector<CkChain> &ch, const std::v
         for (auto &cj : post) cj.n = ncopy;
         copy_list(E, pre, ncopy);
         SweepField<T> *dfl = E.upload(fl, 0);
-        sweep_steps<T>(E, dfl, (int)fl.size(), t0, t1);
+        sweep_steps<T>(E, fl, dfl, t0, t1);
         if (store) copy_list(E, post, ncopy);
     }
 }

@@ -134,4 +134,23 @@ __global__ void __launch_bounds__(4 * NMAX) k1_sweep_dense(const SweepField<T> *
     }
 }
 
+// Whether a launch of nf fields of n points, `steps` contour steps in `blocks`
+// blocks altogether, is faster with k1_sweep_dense than with k_sweep_plane:
+// a block's matrix costs as much as 5 to 50 dense steps, which long blocks pay
+// back and chains of short blocks, or short checkpoint segments, do not.  The
+// times are microseconds per field and, beyond what runs side by side (dense:
+// per SM, by the registers a CTA takes; plane: 10 warps an SM), grow with the
+// fields.  Sweeps measured, plane / dense: 2 fields, 8 blocks of 2 steps: 64
+// points 211 / 109, 128 points 215 / 479; 2 blocks of 50: 1169 / 81, 1198 /
+// 230; 1200 fields, 8 blocks of 2: 425 / 841, 536 / 4408; 2 of 50: 1472 /
+// 583, 2179 / 2119.
+inline bool k1_dense_pays(int n, int nf, long steps, long blocks)
+{
+    const double build = n <= 64 ? 2.0 + n / 6.0 : 0.46 * n, dense_step = n <= 64 ? 0.55 : 1.15;
+    const double plane_step = n <= 32 ? 9.0 : 11.5;
+    const double per_sm = (nf + 147) / 148;
+    const double fd = per_sm * (n <= 32 ? 0.27 : n <= 64 ? 0.62 : 1.0), fp = nf * (n <= 64 ? 1 : 2) / 1480.0;
+    return (blocks * build + steps * dense_step) * (fd > 1 ? fd : 1) < steps * plane_step * (fp > 1 ? fp : 1);
+}
+
 }  // namespace pscfg
