@@ -1966,24 +1966,25 @@ static bool slice_dots_r(Engine &E, const StressJob<T> *dj, int njobs, int maxs)
     return false;
 }
 
-// All jobs of slice_dots with the plane_rx.cuh kernels, in chunks of slices
-// whose spectra take at most 1 GB.
+// All jobs of slice_dots with the plane_rx.cuh kernels, in chunks of jobs and
+// slices whose spectra take at most 1 GB (or one slice of one job).
 template <typename T>
 static bool slice_dots_v(Engine &E, const StressJob<T> *dj, int njobs, int maxs)
 {
     const int ntile = rx3_stress_tiles<T>(E.rx);
-    if (ntile == 0 || 2 * njobs > 65535) return false;
+    if (ntile == 0) return false;
     const size_t per_slice = 2 * (size_t)E.nk * sizeof(cx<T>);
-    const int cs = (int)std::max<size_t>(1, std::min<size_t>((size_t)maxs, ((size_t)1 << 30) / (per_slice * njobs)));
-    if (E.spec_bytes < per_slice * cs * njobs) {
+    const int fit = (int)std::min<size_t>(std::max<size_t>(1, ((size_t)1 << 30) / per_slice), 1 << 30);
+    const int jc = std::min({njobs, fit, 32767}), cs = std::min({maxs, fit / jc, 65535});   // 2 jc and cs: grid limits
+    if (E.spec_bytes < per_slice * cs * jc) {
         E.no_growth_in_capture();
         if (E.spec) cudaFree(E.spec);
         E.spec = nullptr;
         E.spec_bytes = 0;
-        CK(cudaMalloc(&E.spec, per_slice * cs * njobs));
-        E.spec_bytes = per_slice * cs * njobs;
+        CK(cudaMalloc(&E.spec, per_slice * cs * jc));
+        E.spec_bytes = per_slice * cs * jc;
     }
-    const size_t plen = (size_t)cs * njobs * ntile * PSCFG_MAXCP;
+    const size_t plen = (size_t)cs * jc * ntile * PSCFG_MAXCP;
     if (E.stress_part_len < plen) {
         E.no_growth_in_capture();
         if (E.stress_part) cudaFree(E.stress_part);
@@ -1992,11 +1993,14 @@ static bool slice_dots_v(Engine &E, const StressJob<T> *dj, int njobs, int maxs)
         CK(cudaMalloc(&E.stress_part, plen * sizeof(double)));
         E.stress_part_len = plen;
     }
-    for (int s0 = 0; s0 < maxs; s0 += cs) {
-        const int cnt = std::min(cs, maxs - s0);
-        E.launched_n(rx3_stress<T>(E.rx, E.st, dj, njobs, s0, cnt, cs, (cx<T> *)E.spec, E.stress_part));
-        k3_stress_sum_b<T><<<dim3(cnt, njobs), 32, 0, E.st>>>(dj, s0, cs, ntile, E.stress_part);
-        E.launched();
+    for (int j0 = 0; j0 < njobs; j0 += jc) {
+        const int nj = std::min(jc, njobs - j0);
+        for (int s0 = 0; s0 < maxs; s0 += cs) {
+            const int cnt = std::min(cs, maxs - s0);
+            E.launched_n(rx3_stress<T>(E.rx, E.st, dj + j0, nj, s0, cnt, cs, (cx<T> *)E.spec, E.stress_part));
+            k3_stress_sum_b<T><<<dim3(cnt, nj), 32, 0, E.st>>>(dj + j0, s0, cs, ntile, E.stress_part);
+            E.launched();
+        }
     }
     return true;
 }
