@@ -24,6 +24,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <tuple>
 #include <type_traits>
 #include <vector>
 
@@ -163,6 +164,8 @@ struct Engine {
         long launches;
     };
     std::vector<SweepGraph> graphs;
+    using GraphKey = std::tuple<const void *, int, int, int, int, int>;   // as SweepGraph's fields, in their order
+    std::map<GraphKey, int> graph_uses;   // sweeps launched directly so far, of keys that wait for their graph
     // events timing the trial sweeps of the planes-per-CTA choice
     cudaEvent_t tune_e0 = nullptr, tune_e1 = nullptr;
     // optional CUDA-event timing of the phases (ms, accumulated)
@@ -795,10 +798,11 @@ static int sweep_planes(Engine &E, int nf, int n3, int pmax, int tsize, Trial tr
 // Runs emit() -- a fixed sequence of sweep launches whose jobs are read from
 // the descriptors at dfl -- through a CUDA graph captured once per (dfl,
 // field count, step count, precision) and replayed after each descriptor
-// upload (PSCFG_NO_GRAPHS=1 launches directly).
+// upload (PSCFG_NO_GRAPHS=1 launches directly).  The first `direct` sweeps of
+// a key are launched as they are.
 template <typename Emit>
 static void graph_sweep(Engine &E, const void *dfl, int nf, int ns_max, int tsize, int t0, Emit emit,
-                        int variant = 0, cudaEvent_t before = nullptr)
+                        int variant = 0, cudaEvent_t before = nullptr, int direct = 0)
 {
     if (E.no_graphs || E.capturing) {   // inside a captured Anderson iteration: its own nodes
         if (before) CK(cudaEventRecord(before, E.st));
@@ -812,6 +816,13 @@ static void graph_sweep(Engine &E, const void *dfl, int nf, int ns_max, int tsiz
             E.launches += g.launches;
             return;
         }
+    if (direct > 0) {
+        if (E.graph_uses.size() >= 4096) E.graph_uses.clear();
+        if (++E.graph_uses[Engine::GraphKey(dfl, nf, ns_max, tsize, t0, variant)] <= direct) {
+            emit();
+            return;
+        }
+    }
     Engine::SweepGraph sg;
     sg.dfl = dfl;
     sg.nf = nf;
@@ -975,10 +986,14 @@ static bool sweep3v(Engine &E, const SweepField<T> *dfl, int nf, int ns_max, int
         CK(cudaStreamWaitEvent(E.st, E.ev_join, 0));
     };
     // launches longer than their cost on the host need no graph, whose
-    // capture and instantiation (~25 us a launch) the first sweep of an
-    // engine would pay (32^3 x 64: 2448 launches, 65 ms)
+    // capture and instantiation are dear (32^3 x 64: 2448 launches, 65 ms)
     if ((long)std::min(fit, nf) * E.nr >= (1L << 20)) emit();
-    else graph_sweep(E, dfl, nf, ns_max, (int)sizeof(T), t0, emit, 200);
+    // shorter ones only once a key has been used three times: a capture costs
+    // what two or three replays save (density of one instance, 162 launches,
+    // direct / first with its capture / replayed: 8^3 733 / 1185 / 527 us,
+    // 24^3 791 / 1299 / 656), and the keys of a solve whose instances finish
+    // one by one do not come back
+    else graph_sweep(E, dfl, nf, ns_max, (int)sizeof(T), t0, emit, 200, nullptr, 3);
     return true;
 }
 

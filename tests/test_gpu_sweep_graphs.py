@@ -1,0 +1,53 @@
+"""3-D sweeps that are replayed from a CUDA graph once they come again: the
+first pass of an engine pays for no capture, and all passes agree."""
+import time
+
+import numpy as np
+import pytest
+
+from pscf_b200.engine import CHECKPOINT, Engine, FP64
+from tests.cases import diblock, omega_guess
+
+pytestmark = pytest.mark.gpu
+
+
+def first_pass(s, w):
+    times = []
+    for _ in range(8):
+        e = Engine([s], FP64)
+        t = time.perf_counter()
+        e.density(w)
+        times.append(time.perf_counter() - t)
+        e.close()
+    return min(times)
+
+
+# (a capture and the graph's instantiation in the first pass are half as much
+# again as the direct launches; a quarter is timing noise)
+@pytest.mark.parametrize("n", [8, 12, 24])
+def test_the_first_pass_captures_nothing(n, monkeypatch):
+    s = diblock(3, [n] * 3, "orthorhombic", [1.6, 2.1, 1.9], fA=0.35, ds=0.05)
+    w = omega_guess(s, 3, 2.0)[None]
+    t = first_pass(s, w)
+    monkeypatch.setenv("PSCFG_NO_GRAPHS", "1")
+    assert t < 1.25 * first_pass(s, w)
+
+
+@pytest.mark.parametrize("precision", [FP64, FP64 | CHECKPOINT])
+@pytest.mark.parametrize("n", [[12, 10, 14], [32, 32, 32], [64, 64, 4]])
+def test_direct_captured_and_replayed_sweeps_agree(n, precision, monkeypatch):
+    s = diblock(3, n, "orthorhombic", [1.6, 2.1, 1.9], fA=0.35, ds=0.05)
+    w = [np.stack([omega_guess(s, k, 2.0)] * 2) for k in range(6)]
+    e = Engine([s, s], precision)
+    outs, launches = [], []
+    for x in w:
+        before = e.launch_count
+        outs.append(e.density(x)[0])
+        launches.append(e.launch_count - before)
+    e.close()
+    assert len(set(launches)) == 1
+    monkeypatch.setenv("PSCFG_NO_GRAPHS", "1")
+    e = Engine([s, s], precision)
+    for x, rho in zip(w, outs):
+        assert np.array_equal(e.density(x)[0], rho)
+    e.close()
