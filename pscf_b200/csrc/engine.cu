@@ -1006,10 +1006,18 @@ static bool ek_factors_apply(const Engine &E)
     return E.nr >= (1L << 18) && (E.cur == PSCFG_FP32 ? rx3_applies<float>(E) : rx3_applies<double>(E));
 }
 
-// 1-D factors of exp(-lap k^2/6) and exp(-lap k^2/12) (lap = ds b^2) of an
-// orthogonal cell: x (N1/2 + 1), y (N2) and z (N3), each index folded to its
-// minimum image (G_to_bz, src/grid_mod.f90:225-283, along each axis).
-// Appends 2 (N1/2+1+N2+N3).
+// Length of a block's factors: 2 (N1/2+1+N2+N3), in FP32 each with its
+// remainder (EkFactor in plane_rx.cuh).
+template <typename T>
+static size_t ek_factors_len(const Engine &E)
+{
+    return (sizeof(T) == 4 ? 4 : 2) * (size_t)(E.n[0] / 2 + 1 + E.n[1] + E.n[2]);
+}
+
+// Appends the 1-D factors of exp(-lap k^2/6) and exp(-lap k^2/12) (lap = ds
+// b^2) of an orthogonal cell: x (N1/2 + 1), y (N2) and z (N3), each index
+// folded to its minimum image (G_to_bz, src/grid_mod.f90:225-283, along each
+// axis).
 template <typename T>
 static void append_ek_factors(const Engine &E, const Cell &cell, double lap, std::vector<T> &out)
 {
@@ -1020,18 +1028,22 @@ static void append_ek_factors(const Engine &E, const Cell &cell, double lap, std
         const long double g = (long double)cell.G[axis][axis] * kf;
         return g * g;
     };
+    auto add = [&](long double v) {
+        out.push_back((T)v);
+        if (sizeof(T) == 4) out.push_back((T)(v - (long double)(T)v));
+    };
     for (int div : {6, 12}) {
         const long double c = (long double)lap / div;
-        for (int k = 0; k <= M; k++) out.push_back((T)expl(-c * g2(0, k)));
-        for (int k = 0; k < n2; k++) out.push_back((T)expl(-c * g2(1, k)));
-        for (int k = 0; k < n3; k++) out.push_back((T)expl(-c * g2(2, k)));
+        for (int k = 0; k <= M; k++) add(expl(-c * g2(0, k)));
+        for (int k = 0; k < n2; k++) add(expl(-c * g2(1, k)));
+        for (int k = 0; k < n3; k++) add(expl(-c * g2(2, k)));
     }
 }
 
 // The same factors computed on the device from a cell held there (the
 // graph-driven Anderson iteration updates the cell on the device): job j
-// writes 2 (N1/2+1+N2+N3) values from G (row-major 3 x 3, diagonal) and
-// lap.  grid = njobs, 256 threads.
+// writes ek_factors_len values from G (row-major 3 x 3, diagonal) and lap.
+// grid = njobs, 256 threads.
 struct EkfJob {
     const double *G;
     double lap;
@@ -1063,7 +1075,13 @@ static __global__ void k_ek_factors(const EkfJob *jobs, int n1, int n2, int n3)
         }
         const double kf = (k > n / 2) ? (double)(k - n) : (double)k;
         const double g = J.G[axis * 3 + axis] * kf;
-        out[i] = (T)exp(-c * g * g);
+        const double v = exp(-c * g * g);
+        if (sizeof(T) == 8) {
+            out[i] = (T)v;
+        } else {
+            out[2 * i] = (T)v;
+            out[2 * i + 1] = (T)(v - (double)(T)v);
+        }
     }
 }
 
@@ -1200,7 +1218,7 @@ static void run_sweeps(Engine &E, const std::vector<int> &act)
     // (graph-driven iterations: from the cell on the device, k_ek_factors)
     std::vector<T> ekf;
     std::vector<EkfJob> ekj;
-    const int L3 = (int)(E.n[0] / 2 + 1) + E.n[1] + E.n[2];
+    const size_t flen = ek_factors_len<T>(E);
     if (ek_factors_apply(E)) {
         bool ortho = true;
         for (int i : act) {
@@ -1224,7 +1242,7 @@ static void run_sweeps(Engine &E, const std::vector<int> &act)
                         const double kb = I.sys.kuhn[I.sys.block_monomer[c][b]];
                         if (E.amg) {
                             ekj.push_back(EkfJob{E.amg_G[i], I.bds[c][b] * kb * kb, nullptr});
-                            ekf.resize(ekf.size() + 2 * (size_t)L3, (T)0);
+                            ekf.resize(ekf.size() + flen, (T)0);
                         } else {
                             append_ek_factors<T>(E, I.cell, I.bds[c][b] * kb * kb, ekf);
                         }
@@ -1244,9 +1262,9 @@ static void run_sweeps(Engine &E, const std::vector<int> &act)
         T *dtab = E.upload(ekf, off_tab);
         size_t k = 0;
         for (size_t j = 0; j < fl.size(); j += 2)   // fl holds a chain's qf and qr one after the other
-            for (int b = 0; b < fl[j].nblk; b++, k += 2 * (size_t)L3) fl[j].ekf[b] = fl[j + 1].ekf[b] = dtab + k;
+            for (int b = 0; b < fl[j].nblk; b++, k += flen) fl[j].ekf[b] = fl[j + 1].ekf[b] = dtab + k;
         if (!ekj.empty()) {
-            for (size_t j = 0; j < ekj.size(); j++) ekj[j].out = dtab + j * 2 * (size_t)L3;
+            for (size_t j = 0; j < ekj.size(); j++) ekj[j].out = dtab + j * flen;
             EkfJob *dj = E.upload(ekj, off_ekj);
             k_ek_factors<T><<<(unsigned)ekj.size(), 256, 0, E.st>>>(dj, E.n[0], E.n[1], E.n[2]);
             E.launched();
@@ -1538,7 +1556,6 @@ static void ckpt_tables(Engine &E, const std::vector<int> &act, std::vector<cons
     }
     ekf_of.clear();
     std::vector<T> ekf;
-    const int L3 = (int)(E.n[0] / 2 + 1) + E.n[1] + E.n[2];
     bool sep = ek_factors_apply(E);
     for (int i : act)
         for (int a = 0; a < 3; a++)
@@ -1568,7 +1585,7 @@ static void ckpt_tables(Engine &E, const std::vector<int> &act, std::vector<cons
             Inst &I = E.inst[i];
             for (int c = 0; c < I.sys.n_chain; c++) {
                 ekf_of.push_back(dtab + k);
-                k += (size_t)I.sys.n_block[c] * 2 * L3;
+                k += (size_t)I.sys.n_block[c] * ek_factors_len<T>(E);
             }
         }
     }
@@ -1584,7 +1601,6 @@ static void ckpt_segment(Engine &E, const std::vector<CkChain> &ch, const std::v
 {
     const int K = E.ckK;
     const long nr = E.nr;
-    const int L3 = (int)(E.n[0] / 2 + 1) + E.n[1] + E.n[2];
     // qr segments of chains with different ns need different step ranges:
     // one launch group per ns
     std::vector<int> groups;
@@ -1617,7 +1633,7 @@ static void ckpt_segment(Engine &E, const std::vector<CkChain> &ch, const std::v
                 f.eo2[b] = (const T *)I.eo2[c][b];
                 f.ek1[b] = (const T *)I.ek1[c][b];
                 f.ek2[b] = (const T *)I.ek2[c][b];
-                if (!ekf_of.empty()) f.ekf[b] = ekf_of[k] + (size_t)b * 2 * L3;
+                if (!ekf_of.empty()) f.ekf[b] = ekf_of[k] + (size_t)b * ek_factors_len<T>(E);
             }
             const int d = dir > 0 ? 0 : 1;
             f.S1 = (cx<T> *)I.S1[2 * c + d];
