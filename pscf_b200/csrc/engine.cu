@@ -2513,8 +2513,10 @@ static void am_begin(Engine &E, AmRun &R, const pscfg_am_param &prm)
         const double **dwp = (const double **)E.upload(wp, 0);
         UniformJob *duj = E.upload(uj, (wp.size() * sizeof(void *) + 255) / 256 * 256);
         double *part = E.part((size_t)nct * nj);
-        k_partial_sum<double><<<dim3(nct, nj), 256, 0, E.st>>>(dwp, E.nr, part);
-        E.launched();
+        for (int j0 = 0; j0 < nj; j0 += 65535) {
+            k_partial_sum<double><<<dim3(nct, std::min(65535, nj - j0)), 256, 0, E.st>>>(dwp + j0, E.nr, part + (size_t)j0 * nct);
+            E.launched();
+        }
         k_final_sum<<<(unsigned)((nj + 3) / 4), 128, 0, E.st>>>(part, nct, (double)E.nr, E.d_small, nj);
         E.launched();
         k_omega_uniform<<<dim3(red_ctas(E.nr, ninst), ninst), 256, 0, E.st>>>(duj, E.nr);
