@@ -363,12 +363,13 @@ long pscfg_steps_per_density(const pscfg_engine *e);
 long pscfg_launch_count(const pscfg_engine *e);
 
 /* Planes per CTA that the 3-D sweep of this engine's grid (16^3, 32^3) uses
- * for n_fields fields in FP64 (fp32 != 0: FP32).  FP64: by the launch size.
- * FP32, and FP64 with PSCFG_PLANES set: as measured by the engine for its
- * register sweep (one timed trial sweep per candidate before the first real
- * sweep of each class of field counts -- up to the same power of two -- the
- * fastest kept for the process); -1 when the thread-block-cluster sweep
- * (32^3, FP64) was the fastest; 0 while undecided or for other grids. */
+ * for n_fields fields in FP64 (fp32 != 0: FP32).  FP64 at 32^3: by the launch
+ * size.  16^3, and FP32 at 32^3: as measured by the engine for its register
+ * sweep (one timed trial sweep per candidate before the first real sweep of
+ * each class of field counts -- up to the same power of two -- the fastest
+ * kept for the process); 0 while undecided.  With PSCFG_PLANES set: the count
+ * it forces (-1: the thread-block-cluster sweep, FP64 at 32^3).  0 for other
+ * grids. */
 int pscfg_sweep_planes(const pscfg_engine *e, int n_fields, int fp32);
 
 #ifdef __cplusplus

@@ -757,15 +757,20 @@ static long planes_key(int n3, int tsize, int nf)
     return ((long)n3 * 16 + tsize) * 100000 + b;
 }
 
+// the count that PSCFG_PLANES forces (pmax, pmax/2, ..., 1), or 0
+static int forced_planes(int planes, int pmax)
+{
+    for (int p = pmax; p >= 1; p /= 2)
+        if (planes == p) return p;
+    return 0;
+}
+
 // trial(p, e0, e1) enqueues one sweep with p planes per CTA, recording e0
 // just before its first launch and e1 after its last.
 template <typename Trial>
 static int sweep_planes(Engine &E, int nf, int n3, int pmax, int tsize, Trial trial, bool cluster = false)
 {
-    if (E.planes > 0) {
-        for (int p = pmax; p >= 1; p /= 2)
-            if (E.planes == p) return p;
-    }
+    if (const int p = forced_planes(E.planes, pmax)) return p;
     if (E.planes < 0 && cluster) return 0;   // PSCFG_PLANES=-1: the cluster sweep
     const long key = planes_key(n3, tsize, nf);
     {
@@ -4774,6 +4779,8 @@ int pscfg_sweep_planes(const pscfg_engine *e, int n_fields, int fp32)
     const int n3 = e->E.n[2];
     if (n3 != 16 && n3 != 32) return 0;
     if (!fp32 && rx3_applies<double>(e->E)) return rx3_planes<double>(e->E.rx, (n_fields + 1) / 2);
+    if (const int p = forced_planes(e->E.planes, n3 == 32 ? 4 : 8)) return p;
+    if (e->E.planes < 0 && n3 == 32 && !fp32) return -1;
     const long key = planes_key(n3, fp32 ? 4 : 8, n_fields);
     std::lock_guard<std::mutex> lk(g_planes_mu);
     auto it = g_planes_best.find(key);
