@@ -341,12 +341,18 @@ struct Engine {
         }
         return d_part;
     }
-    // n kernels queued by a sweep_rx.h launch function (n < 0: one failed)
+    // n kernels queued by a sweep_rx.h launch function (n < 0: one failed;
+    // 0: the grid has no such kernels)
     bool launched_n(int n)
     {
         launched();
         launches += n - 1;
         return n > 0;
+    }
+    // the same where the grid is known to have them (rx3_applies)
+    void must_launch(int n)
+    {
+        if (!launched_n(n)) throw Err(PSCFG_ECUDA, "a step's kernels were not launched");
     }
     void launched(cudaError_t e = cudaGetLastError())
     {
@@ -970,7 +976,7 @@ static bool sweep3v(Engine &E, const SweepField<T> *dfl, int nf, int ns_max, int
     const long field_bytes = (long)sizeof(T) * (4 * E.nk + 3 * E.nr);
     const int fit = (int)std::max<long>(2, ((long)80 << 20) / field_bytes);
     auto step = [&](const SweepField<T> *d, int n, cudaStream_t st, int t) {
-        E.launched_n(t < t0 ? rx3_first<T>(E.rx, st, d, n, t0) : rx3_step<T>(E.rx, st, d, n, t));
+        E.must_launch(t < t0 ? rx3_first<T>(E.rx, st, d, n, t0) : rx3_step<T>(E.rx, st, d, n, t));
     };
     auto emit = [&]() {
         if (nf < 2 || E.no_branch) {
@@ -2033,7 +2039,7 @@ static bool slice_dots_v(Engine &E, const StressJob<T> *dj, int njobs, int maxs)
         const int nj = std::min(jc, njobs - j0);
         for (int s0 = 0; s0 < maxs; s0 += cs) {
             const int cnt = std::min(cs, maxs - s0);
-            E.launched_n(rx3_stress<T>(E.rx, E.st, dj + j0, nj, s0, cnt, cs, (cx<T> *)E.spec, E.stress_part));
+            E.must_launch(rx3_stress<T>(E.rx, E.st, dj + j0, nj, s0, cnt, cs, (cx<T> *)E.spec, E.stress_part));
             k3_stress_sum_b<T><<<dim3(cnt, nj), 32, 0, E.st>>>(dj + j0, s0, cs, ntile, E.stress_part);
             E.launched();
         }
@@ -3207,8 +3213,8 @@ static void run_single_steps(Engine &E, const SweepField<T> *dfl, int nf)
     const PlaneGeom &g = E.geom();
     const long nr = E.nr;
     if (rx3_applies<T>(E)) {
-        E.launched_n(rx3_first<T>(E.rx, E.st, dfl, nf, 0));
-        E.launched_n(rx3_step<T>(E.rx, E.st, dfl, nf, 0));
+        E.must_launch(rx3_first<T>(E.rx, E.st, dfl, nf, 0));
+        E.must_launch(rx3_step<T>(E.rx, E.st, dfl, nf, 0));
         return;
     }
     if (E.dim <= 2) {
@@ -3500,8 +3506,8 @@ static void adjoint_impl(Engine &E, const std::vector<int> &act, const std::vect
         if (half && nl > 0) {
             CK(cudaEventRecord(E.ev_fork, E.st));
             CK(cudaStreamWaitEvent(E.st2, E.ev_fork, 0));
-            E.launched_n(rx3_first<T>(E.rx, E.st2, dfl + nl, (int)flq.size(), 0));
-            E.launched_n(rx3_half<T>(E.rx, E.st2, dfl + nl, (int)flq.size()));
+            E.must_launch(rx3_first<T>(E.rx, E.st2, dfl + nl, (int)flq.size(), 0));
+            E.must_launch(rx3_half<T>(E.rx, E.st2, dfl + nl, (int)flq.size()));
             CK(cudaEventRecord(E.ev_join, E.st2));
             run_single_steps<T>(E, dfl, nl);
             CK(cudaStreamWaitEvent(E.st, E.ev_join, 0));
