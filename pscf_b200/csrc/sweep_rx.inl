@@ -146,11 +146,15 @@ template <typename T, typename F> static int with_line(const RxPlan &p, int nf, 
     return f(p.z, RxInt<16>(), RxInt<256>(), RxInt<2>());
 }
 
-// the same for the stress pass, whose two tiles have to leave room for several
-// CTAs per SM
+// The same for the stress pass, which holds two tiles: 8 columns where tiles of
+// 16 would leave one CTA to an SM (a 64 x 128 x 224 FP64 solve's z pass: 8.2 ms
+// with 16, 6.0 with 8).
 template <typename T, typename F> static int with_stress_line(const RxPlan &p, F f)
 {
-    if (p.z.n3 == 224 && sizeof(T) == 8) return f(RzFixed<224, 16>(), RxInt<8>(), RxInt<128>(), RxInt<3>());
+    if (2 * rz_smem<T>(p.n3, 16, 2) > SMEM_MOST) {
+        if (p.z.n3 == 224) return f(RzFixed<224, 16>(), RxInt<8>(), RxInt<128>(), RxInt<3>());
+        return f(p.z, RxInt<8>(), RxInt<128>(), RxInt<3>());
+    }
     return with_line<T>(p, 1 << 20, f);
 }
 
