@@ -1533,11 +1533,12 @@ static void slice_dots(Engine &E, const std::vector<StressJob<T>> &jobs);
 // recomputed from its checkpoint into segA (qf, upward) or segB (qr,
 // downward) by the ordinary sweep kernels, through descriptors whose slab
 // points K slices before the segment buffer (step_slices indexes the
-// absolute slice).  A recomputed segment repeats the checkpointing pass's
-// operations exactly, so it equals the slices that pass produced; against
-// an uninterrupted sweep the slices agree to the last bits (a segment's
-// first step starts from the checkpoint in global memory, where the fused
-// sweep kernels carry it over from the previous step).
+// absolute slice).  A recomputed segment agrees with the slices of the
+// checkpointing pass, and those with an uninterrupted sweep's, to the last
+// bits (a segment's first step starts from the checkpoint in global memory,
+// where the fused sweep kernels carry it over from the previous step; with
+// other numbers of fields or steps a 1-D or 2-D grid may take another of its
+// kernels).
 struct CkChain {
     int inst, c;
 };

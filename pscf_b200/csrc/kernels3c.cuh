@@ -748,58 +748,6 @@ __global__ void __launch_bounds__(128, 4) k3r_stress_xy(const StressJob<T> *job,
     PSk::forward_to(buf, spec + ((long)blockIdx.y * 2 + blockIdx.z) * nk + (long)z0 * PSk::PS);
 }
 
-// Pass 2: one thread per z column: z-forward of the qf spectrum in
-// registers (written back in place), then of the qr spectrum, and the
-// weighted products sum_k wdgsq_b(k) Re(F conj R) of its column; block
-// sums per tile of 128 columns.  grid = (ceil(P/128), cs).
-template <typename T, int N1, int N2, int N3>
-__global__ void __launch_bounds__(128) k3r_stress_z(const StressJob<T> *job, int s0, cx<T> *spec, double *part)
-{
-    constexpr int NH = N1 / 2 + 1, P = N2 * NH;
-    const StressJob<T> &J = *job;
-    const int s = s0 + blockIdx.y;
-    if (s >= J.nslices) return;
-    __shared__ double red[32];
-    const long nk = (long)P * N3;
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    double acc[PSCFG_MAXCP] = {0, 0, 0, 0, 0, 0};
-    if (col < P) {
-        cx<T> *sf = spec + ((long)blockIdx.y * 2) * nk + col;
-        const cx<T> *sr = sf + nk;
-        cx<T> v[N3];
-#pragma unroll
-        for (int z = 0; z < N3; z++) v[z] = sf[(long)z * P];
-        RegDft<N3, -1, T>::run(v);
-#pragma unroll
-        for (int k = 0; k < N3; k++) sf[(long)k * P] = v[k];
-        // re-read the stored spectrum below instead of keeping it live in
-        // registers next to the second column (which would spill)
-        asm volatile("" ::: "memory");
-#pragma unroll
-        for (int z = 0; z < N3; z++) v[z] = sr[(long)z * P];
-        RegDft<N3, -1, T>::run(v);
-        double d[N3];
-#pragma unroll
-        for (int k = 0; k < N3; k++) {
-            const cx<T> f = sf[(long)k * P];
-            d[k] = (double)f.x * (double)v[k].x + (double)f.y * (double)v[k].y;
-        }
-        const double *w = J.wdgsq + col;
-#pragma unroll 1
-        for (int b = 0; b < J.ncp; b++) {
-            double a = 0.0;
-#pragma unroll
-            for (int k = 0; k < N3; k++) a += __ldg(w + (long)b * nk + (long)k * P) * d[k];
-            acc[b] = a;
-        }
-    }
-    for (int b = 0; b < J.ncp; b++) {
-        const double tot = block_sum(acc[b], red);
-        if (threadIdx.x == 0) part[((long)blockIdx.y * gridDim.x + blockIdx.x) * PSCFG_MAXCP + b] = tot;
-        __syncthreads();
-    }
-}
-
 // Stress pass 2 with two lanes per z column (as k3s_zconv): each lane ends
 // with half of the qf spectrum and the same half of the qr spectrum in
 // registers and forms its products sum_k wdgsq_b(k) Re(F conj R) there;
