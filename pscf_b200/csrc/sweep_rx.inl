@@ -277,7 +277,6 @@ int rx3_stress(const RxPlan &p, cudaStream_t st, const StressJob<T> *jobs, int n
     template int rx3_planes<T>(const RxPlan &, int);                                                                 \
     template bool rx3_fits<T>(const RxPlan &);                                                                       \
     template int rx3_first<T>(const RxPlan &, cudaStream_t, const SweepField<T> *, int, int);                        \
-    template int rx3_half<T>(const RxPlan &, cudaStream_t, const SweepField<T> *, int);                              \
     template int rx3_step<T>(const RxPlan &, cudaStream_t, const SweepField<T> *, int, int);                         \
     template int rx3_stress_tiles<T>(const RxPlan &);                                                                \
     template int rx3_stress<T>(const RxPlan &, cudaStream_t, const StressJob<T> *, int, int, int, int, cx<T> *, double *);

@@ -4,5 +4,6 @@
 namespace pscfg {
 
 RX3_INSTANCES(double)
+template int rx3_half<double>(const RxPlan &, cudaStream_t, const SweepField<double> *, int);   // (the adjoint: FP64 alone)
 
 }  // namespace pscfg
