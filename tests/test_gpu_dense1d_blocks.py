@@ -35,24 +35,31 @@ def test_short_blocks_match_oracle(n, steps, count):
             assert rel_err(rho[i], rho_ref) < 1e-12
 
 
-def sweep_ms(s, w, count):
-    e = Engine([s] * count, FP64)
-    e.set_profiling(True)
-    times = []
-    for _ in range(15):
-        before = e.profile()["sweep_ms"]
-        e.density(w)
-        times.append(e.profile()["sweep_ms"] - before)
-    e.close()
-    return min(times)
+def sweep_ms(e, w):
+    before = e.profile()["sweep_ms"]
+    e.density(w)
+    return e.profile()["sweep_ms"] - before
 
 
-# A quarter above the other kernel is timing noise; the dense step takes 2.2
-# (one instance) to 4 times as long here (96).
+# A quarter above the other kernel is timing noise, of the least of both
+# sides' sweeps, taken in turn; the dense step takes 2.2 (one instance) to 4
+# times as long here (96).
 @pytest.mark.parametrize("n,count", [(128, 1), (128, 96), (70, 96)])
 def test_short_blocks_are_not_slower_than_the_general_kernel(n, count, monkeypatch):
     s = multiblock(n, 2)
     w = np.stack([omega_guess(s, 3, 2.0)] * count)
-    t = sweep_ms(s, w, count)
+    e = Engine([s] * count, FP64)
     monkeypatch.setenv("PSCFG_GENERIC_KERNELS", "1")
-    assert t < 1.25 * sweep_ms(s, w, count)
+    g = Engine([s] * count, FP64)
+    times, general = [], []
+    for x in (e, g):
+        x.set_profiling(True)
+        x.density(w)
+    for _ in range(60):
+        times.append(sweep_ms(e, w))
+        general.append(sweep_ms(g, w))
+        if len(times) >= 15 and min(times) < 1.25 * min(general):
+            break
+    e.close()
+    g.close()
+    assert min(times) < 1.25 * min(general)

@@ -12,25 +12,30 @@ pytestmark = pytest.mark.gpu
 
 
 def first_pass(s, w):
-    times = []
-    for _ in range(8):
-        e = Engine([s], FP64)
-        t = time.perf_counter()
-        e.density(w)
-        times.append(time.perf_counter() - t)
-        e.close()
-    return min(times)
+    e = Engine([s], FP64)
+    t = time.perf_counter()
+    e.density(w)
+    t = time.perf_counter() - t
+    e.close()
+    return t
 
 
 # (a capture and the graph's instantiation in the first pass are half as much
-# again as the direct launches; a quarter is timing noise)
+# again as the direct launches; a quarter is timing noise, of the least of
+# both sides' passes, taken in turn)
 @pytest.mark.parametrize("n", [8, 12, 24])
 def test_the_first_pass_captures_nothing(n, monkeypatch):
     s = diblock(3, [n] * 3, "orthorhombic", [1.6, 2.1, 1.9], fA=0.35, ds=0.05)
     w = omega_guess(s, 3, 2.0)[None]
-    t = first_pass(s, w)
-    monkeypatch.setenv("PSCFG_NO_GRAPHS", "1")
-    assert t < 1.25 * first_pass(s, w)
+    graphs, direct = [], []
+    for _ in range(30):
+        monkeypatch.delenv("PSCFG_NO_GRAPHS", raising=False)
+        graphs.append(first_pass(s, w))
+        monkeypatch.setenv("PSCFG_NO_GRAPHS", "1")
+        direct.append(first_pass(s, w))
+        if len(graphs) >= 8 and min(graphs) < 1.25 * min(direct):
+            break
+    assert min(graphs) < 1.25 * min(direct)
 
 
 @pytest.mark.parametrize("precision", [FP64, FP64 | CHECKPOINT])
